@@ -387,8 +387,9 @@ int phmm_fb1d_emissions(const phmm_model_desc *model, int32_t n_pairs, const int
  * With the batch's cell_mask set, a nonzero byte marks a cell inside the
  * envelope of beam_viterbi_2d (dp/hmm_beam.py:397-490): a state whose cell
  * or predecessor cell lies outside keeps NEG_INF and points to the origin.
- * Scratch from the caller's workspace (phmm_viterbi_workspace_bytes:
- * three diagonals and one backpointer byte per cell and state). */
+ * Scratch from the caller's workspace (phmm_viterbi_workspace_bytes: one
+ * backpointer byte per cell and emitting state, and the last row of every 8 to 64
+ * rows in float64). */
 int phmm_viterbi_workspace_bytes(const phmm_model_desc *model, const phmm_batch *batch, size_t *bytes);
 int phmm_viterbi(const phmm_model_desc *model, const phmm_batch *batch, const double *log_chi,
                  const double *log_emit_M, const double *log_emit_I, const double *log_emit_D,
@@ -407,7 +408,8 @@ int phmm_viterbi(const phmm_model_desc *model, const phmm_batch *batch, const do
  * (i, j, state) from (0, 0, S) on, sample s of pair p at triple
  * n_samples * sum_{q<p} (Lx_q+Ly_q+1) + s (Lx_p+Ly_p+1), path_len
  * [P][n_samples], status [P].  N <= 64.  Scratch (phmm_sample_workspace_bytes):
- * the forward tables, (Lx+1)(Ly+1)N doubles per pair. */
+ * the forward tables, (Lx+1)(Ly+1)N doubles per pair, the linear tables and the
+ * last row of every 8 to 32 rows. */
 int phmm_sample_workspace_bytes(const phmm_model_desc *model, const phmm_batch *batch, size_t *bytes);
 int phmm_sample_paths(const phmm_model_desc *model, const phmm_batch *batch, const double *log_chi,
                       const double *log_emit_M, const double *log_emit_I, const double *log_emit_D,
