@@ -3,12 +3,24 @@
 // Along a fixed alignment the pair HMM is an ordinary HMM over the alignment
 // columns (dp/hmm.py:127-250, 471-607): column l emits through the states of
 // its type only (dp/hmm.py:854-1082), alpha_l = (alpha_{l-1} chi) .* e_l.
-// One CTA per pair walks its columns: thread k owns destination k, chi is
-// staged in shared memory with an odd row stride (row and column walks are
-// both conflict-free), every alpha / beta vector is rescaled by a power of
-// two after its step (exact, the exponents kept as integers), and the
-// expected transition counts accumulate during the backward walk in
-// Kahan-compensated float32 in shared memory, one entry per thread slot.
+// One CTA per pair, in two phases:
+//   recursions   one warp walks the columns forward and another backward at the
+//                same time; a lane owns one state (two above 32) with its column
+//                or row of chi in registers, the vector passes through shared
+//                memory, and the power-of-two rescaling after every column
+//                (exact, the exponents kept as integers) takes its maximum by one
+//                warp reduction: no barrier, about 200 clocks a column;
+//   counts       every thread owns entries of the expected transitions, in
+//                Kahan-compensated float32 registers, and walks the columns from
+//                the last to the first through tiles of both vectors in shared
+//                memory (the order of an entry's additions is that of the
+//                backward walk, so the sums do not depend on the split).
+// What bounds it is the recursions' chain: column by column a product of N
+// multiply-adds, a maximum and a rescaling.  With one 128-thread CTA walking the
+// columns forward, then backward and counting every pair of states between its
+// barriers (each thread taking the float64 exponential of the column's scale),
+// 256 alignments of 40-500 columns took 1.51 ms at 17 states; now 0.18 ms, and 64 of
+// 60-400 at 42 states 0.26 ms instead of 1.99, with the same bits.
 // Emission tables come as linear per-column rows [sum L][N]; a second
 // kernel builds them from an alignment and the per-group tables the 2D path
 // uses.
@@ -16,6 +28,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -24,8 +37,8 @@ extern "C" __attribute__((visibility("hidden"))) void phmm_internal_set_error(co
 
 namespace fb1 {
 
-constexpr int NT = 128;          // threads per pair
-constexpr int MAXN = 64;         // states (chi and the count accumulators in shared memory)
+constexpr int MAXN = 64;         // states
+constexpr int TILE = 16;         // columns staged for the counts at a time
 constexpr int EXPN = -(1 << 28); // exponent of an all-zero vector
 constexpr double LN2 = 0.69314718055994530942;
 
@@ -41,169 +54,256 @@ __device__ __forceinline__ int exp2_of(float m) {   // m * 2^-e in [0.5, 1) for 
     return e;
 }
 
-__device__ float block_max(float v, float *red) {
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    float m = red[0];
-    for (int w = 1; w < NT / 32; ++w) m = fmaxf(m, red[w]);
-    return m;
+// The largest of the warp's values and 0 (compared as integers: the values are not negative).
+__device__ __forceinline__ float warp_max(float v) {
+    return __int_as_float(__reduce_max_sync(0xffffffffu, max(__float_as_int(v), 0)));
 }
 
-__device__ double block_sum_d(double v, double *red) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    double s = 0.0;
-    for (int w = 0; w < NT / 32; ++w) s += red[w];
-    return s;
+// v * 2^-e
+__device__ __forceinline__ float scale_down(float v, int e) {
+    return (e >= -126 && e <= 126) ? v * __int_as_float((127 - e) << 23) : ldexpf(v, -e);
 }
 
-// shared layout: chi [N][NP] (NP = N | 1), a/b/w vectors, count sums and compensations
+// Rescales a vector held NR states to a lane by the power of two of its largest
+// entry; returns the exponent, cum plus its own (EXPN once a vector is all zero).
+template <int NR>
+__device__ __forceinline__ int rescale(float (&v)[NR], int cum) {
+    float mx = v[0];
+    if (NR > 1) mx = fmaxf(mx, v[NR - 1]);
+    mx = warp_max(mx);
+    const int b = __float_as_int(mx) >> 23;
+    const int e = mx > 0.f ? (b > 0 && b < 255 ? b - 126 : exp2_of(mx)) : 0;
+#pragma unroll
+    for (int z = 0; z < NR; ++z) v[z] = mx > 0.f ? scale_down(v[z], e) : 0.f;
+    return (mx > 0.f && cum > EXPN) ? cum + e : EXPN;
+}
+
+struct Args {
+    const Meta *meta;
+    int N, chi_per_pair, init, fin;
+    const float *chi, *emit;
+    float *alpha, *beta;    // rescaled vectors by column
+    int *aexp, *bexp;       // their exponents
+    double *ll, *n;
+    float *post;
+    int32_t *status;
+};
+
+// The dot products of a lane's NR states: c[z][.] against the vector in shared
+// memory (padded with zeros to NB), one term after the other.
+template <int NB, int NR>
+__device__ __forceinline__ void dots(const float *vec, const float (&c)[NR][NB], float (&s)[NR]) {
+#pragma unroll
+    for (int z = 0; z < NR; ++z) s[z] = 0.f;
+#pragma unroll
+    for (int j4 = 0; j4 < NB / 4; ++j4) {
+        const float4 f = ((const float4 *)vec)[j4];
+#pragma unroll
+        for (int z = 0; z < NR; ++z) {
+            s[z] = fmaf(f.x, c[z][4 * j4], s[z]);
+            s[z] = fmaf(f.y, c[z][4 * j4 + 1], s[z]);
+            s[z] = fmaf(f.z, c[z][4 * j4 + 2], s[z]);
+            s[z] = fmaf(f.w, c[z][4 * j4 + 3], s[z]);
+        }
+    }
+}
+
+// NB: bound of N (a multiple of 4); NR: states per lane of the recursions; NT:
+// threads; EPT: entries of the counts per thread (EPT NT >= NB NB).
+template <int NB, int NR, int NT, int EPT>
 __global__ void __launch_bounds__(NT)
-fb1d_kernel(const Meta *__restrict__ meta, int N, const float *__restrict__ chi_all, int chi_per_pair,
-            const float *__restrict__ emit, int init_state, int final_state, float *__restrict__ alpha,
-            int *__restrict__ aexp, double *__restrict__ ll_out, double *__restrict__ n_out,
-            float *__restrict__ post, int32_t *__restrict__ status) {
-    extern __shared__ float smf[];
-    __shared__ float redf[NT / 32];
-    __shared__ double redd[NT / 32];
-    const int p = blockIdx.x, tid = threadIdx.x;
-    const Meta m = meta[p];
-    const int NP = N | 1;
-    float *chi = smf;                 // [N][NP]
-    float *va = chi + N * NP;         // [N] current vector
-    float *vw = va + MAXN;            // [N] work vector
-    float *cs = vw + MAXN;            // [N*N] count sums
-    float *cc = cs + MAXN * MAXN;     // [N*N] count compensations
-    const float *chig = chi_all + (chi_per_pair ? (int64_t)p * N * N : 0);
-    for (int idx = tid; idx < N * N; idx += NT) {
-        chi[(idx / N) * NP + idx % N] = chig[idx];
-        cs[idx] = 0.f;
-        cc[idx] = 0.f;
-    }
+fb1d_kernel(const __grid_constant__ Args A) {
+    constexpr int AHEAD = 4;                    // columns the emissions are loaded ahead
+    static_assert(EPT * NT >= NB * NB, "every entry has a thread");
+    extern __shared__ float smf[];              // chi [N][N], then two tiles [TILE][N] of both vectors
+    __shared__ __align__(16) float vec[2][2][NB];   // direction, column parity
+    __shared__ float scale[2][TILE];            // 2^(exponents - log2 P) of the transitions, of the posteriors
+    __shared__ double s_lp2;
+    __shared__ int s_ok;
+    __shared__ float s_f[2];                    // scales of the last column's alpha and the first's beta
+    const int p = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const Meta m = A.meta[p];
+    const int N = A.N, NN = N * N, L = m.L;
+    float *chi = smf;
+    const float *chig = A.chi + (A.chi_per_pair ? (int64_t)p * NN : 0);
+    for (int idx = tid; idx < NN; idx += NT) chi[idx] = chig[idx];
+    double *nt = A.n + (int64_t)p * NN;
     __syncthreads();
-    const int L = m.L;
-    double *nt = n_out + (int64_t)p * N * N;
     if (L == 0) {   // empty alignment: S -> E directly
-        const float c = chi[init_state * NP + final_state];
+        const float c = chi[A.init * N + A.fin];
         if (tid == 0) {
-            ll_out[p] = c > 0.f ? log((double)c) : -1e30;
-            if (!(c > 0.f)) atomicOr(status + p, PHMM_ST_ZERO_LL);
+            A.ll[p] = c > 0.f ? log((double)c) : -1e30;
+            if (!(c > 0.f)) atomicOr(A.status + p, PHMM_ST_ZERO_LL);
         }
-        for (int idx = tid; idx < N * N; idx += NT) nt[idx] = (idx == init_state * N + final_state) ? 1.0 : 0.0;
+        for (int idx = tid; idx < NN; idx += NT) nt[idx] = (idx == A.init * N + A.fin) ? 1.0 : 0.0;
         return;
     }
-    const float *em = emit + m.off * N;
-    float *al = alpha + m.off * N;
-    int *ae = aexp + m.off;
-    // ---- forward
-    int cum = 0;
-    for (int l = 0; l < L; ++l) {
-        float mx = 0.f;
-        for (int k = tid; k < N; k += NT) {
-            float s = 0.f;
-            if (l == 0) {
-                s = chi[init_state * NP + k];
-            } else {
-                for (int j = 0; j < N; ++j) s = fmaf(va[j], chi[j * NP + k], s);
+    const float *em = A.emit + m.off * N;
+    float *al = A.alpha + m.off * N, *be = A.beta + m.off * N;
+    int *ae = A.aexp + m.off, *bx = A.bexp + m.off;
+
+    if (warp < 2) {
+        // ---- the recursions: warp 0 forward, warp 1 backward
+        const bool fwd = warp == 0;
+        float c[NR][NB], v[NR], w[NR];
+        int k[NR];
+#pragma unroll
+        for (int z = 0; z < NR; ++z) {
+            k[z] = lane + 32 * z;
+#pragma unroll
+            for (int j = 0; j < NB; ++j)
+                c[z][j] = (k[z] < N && j < N) ? (fwd ? chi[j * N + k[z]] : chi[k[z] * N + j]) : 0.f;
+        }
+        auto put = [&](int par, const float (&x)[NR]) {   // the vector into shared memory
+#pragma unroll
+            for (int z = 0; z < NR; ++z)
+                if (k[z] < NB) vec[warp][par][k[z]] = x[z];
+            __syncwarp();
+        };
+        auto load = [&](const float *row, bool in, float (&x)[NR]) {
+#pragma unroll
+            for (int z = 0; z < NR; ++z) x[z] = (in && k[z] < N) ? __ldg(row + k[z]) : 0.f;
+        };
+        float e[AHEAD][NR];
+        int cum;
+        if (fwd) {
+#pragma unroll
+            for (int u = 0; u < AHEAD; ++u) load(em + (int64_t)u * N, u < L, e[u]);
+            cum = 0;
+            for (int l0 = 0; l0 < L; l0 += AHEAD) {
+#pragma unroll
+                for (int u = 0; u < AHEAD; ++u) {
+                    const int l = l0 + u;
+                    if (l >= L) break;
+                    if (l == 0) {
+#pragma unroll
+                        for (int z = 0; z < NR; ++z) v[z] = k[z] < N ? chi[A.init * N + k[z]] : 0.f;
+                    } else {
+                        dots<NB, NR>(vec[0][l & 1], c, v);
+                    }
+#pragma unroll
+                    for (int z = 0; z < NR; ++z) v[z] = v[z] * e[u][z];
+                    load(em + (int64_t)(l + AHEAD) * N, l + AHEAD < L, e[u]);
+                    cum = rescale<NR>(v, cum);
+                    put((l + 1) & 1, v);
+#pragma unroll
+                    for (int z = 0; z < NR; ++z)
+                        if (k[z] < N) al[(int64_t)l * N + k[z]] = v[z];
+                    if (lane == 0) ae[l] = cum;
+                }
             }
-            const float v = s * em[(int64_t)l * N + k];
-            vw[k] = v;
-            mx = fmaxf(mx, v);
+            double pz = 0.0, part[NR];
+#pragma unroll
+            for (int z = 0; z < NR; ++z) {
+                part[z] = k[z] < N ? (double)v[z] * (double)chi[k[z] * N + A.fin] : 0.0;
+                for (int o = 16; o > 0; o >>= 1) part[z] += __shfl_xor_sync(0xffffffffu, part[z], o);
+                pz += part[z];
+            }
+            const bool ok = pz > 0.0 && cum > EXPN;
+            if (lane == 0) {
+                const double lp2 = ok ? log2(pz) + (double)cum : 0.0;   // log2 P
+                s_lp2 = lp2;
+                s_ok = ok;
+                A.ll[p] = ok ? lp2 * LN2 : -1e30;
+                if (!ok) atomicOr(A.status + p, PHMM_ST_ZERO_LL);
+            }
+        } else {
+#pragma unroll
+            for (int u = 0; u < AHEAD; ++u) load(em + (int64_t)(L - 1 - u) * N, L - 1 - u >= 0, e[u]);
+#pragma unroll
+            for (int z = 0; z < NR; ++z) v[z] = k[z] < N ? chi[k[z] * N + A.fin] : 0.f;
+            cum = rescale<NR>(v, 0);
+            for (int l0 = L - 1; l0 >= 0; l0 -= AHEAD) {
+#pragma unroll
+                for (int u = 0; u < AHEAD; ++u) {
+                    const int l = l0 - u;       // v = b_l
+                    if (l < 0) break;
+#pragma unroll
+                    for (int z = 0; z < NR; ++z)
+                        if (k[z] < N) be[(int64_t)l * N + k[z]] = v[z];
+                    if (lane == 0) bx[l] = cum;
+#pragma unroll
+                    for (int z = 0; z < NR; ++z) w[z] = e[u][z] * v[z];
+                    load(em + (int64_t)(l - AHEAD) * N, l - AHEAD >= 0, e[u]);
+                    if (l == 0) break;
+                    put(l & 1, w);
+                    dots<NB, NR>(vec[1][l & 1], c, v);   // b_{l-1}
+                    cum = rescale<NR>(v, cum);
+                }
+            }
         }
-        mx = block_max(mx, redf);   // (barriers: every vw written, every va read)
-        const int e = mx > 0.f ? exp2_of(mx) : 0;
-        for (int k = tid; k < N; k += NT) {
-            const float v = mx > 0.f ? ldexpf(vw[k], -e) : 0.f;
-            va[k] = v;
-            al[(int64_t)l * N + k] = v;
-        }
-        cum = (mx > 0.f && cum > EXPN) ? cum + e : EXPN;
-        if (tid == 0) ae[l] = cum;
-        __syncthreads();
     }
-    double pz = 0.0;
-    for (int k = tid; k < N; k += NT) pz += (double)va[k] * (double)chi[k * NP + final_state];
-    pz = block_sum_d(pz, redd);
-    const bool ok = pz > 0.0 && cum > EXPN;
-    const double lp2 = ok ? log2(pz) + (double)cum : 0.0;   // log2 P
-    if (tid == 0) {
-        ll_out[p] = ok ? lp2 * LN2 : -1e30;
-        if (!ok) atomicOr(status + p, PHMM_ST_ZERO_LL);
-    }
-    if (!ok) {
-        for (int idx = tid; idx < N * N; idx += NT) nt[idx] = 0.0;
+    __syncthreads();
+    if (!s_ok) {
+        for (int idx = tid; idx < NN; idx += NT) nt[idx] = 0.0;
         return;
     }
-    // ---- backward, with the counts
-    auto add = [&](int idx, float v) {   // Kahan
-        const float y = v - cc[idx];
-        const float t = cs[idx] + y;
-        cc[idx] = (t - cs[idx]) - y;
-        cs[idx] = t;
+    // ---- the counts
+    const double lp2 = s_lp2;
+    float *ta = smf + NN, *tw = ta + TILE * N;  // a_l and w_{l+1} = e_{l+1} b_{l+1} of the tile's columns
+    if (tid < 2) s_f[tid] = (float)exp2((double)(tid == 0 ? ae[L - 1] : bx[0]) - lp2);
+    __syncthreads();
+    float ch[EPT], cs[EPT], cc[EPT];
+    int es[EPT], ek[EPT];
+    auto add = [&](float &s, float &c, float v, float f) {   // Kahan, of the product v f
+        const float y = fmaf(v, f, -c), t = s + y;
+        c = (t - s) - y;
+        s = t;
     };
-    // terminal: n[s][final] += a_{L-1}[s] chi[s][final] / P; b_{L-1}[s] = chi[s][final]
-    {
-        const float f = (float)exp2((double)ae[L - 1] - lp2);
-        for (int s = tid; s < N; s += NT) add(s * N + final_state, al[(int64_t)(L - 1) * N + s] * chi[s * NP + final_state] * f);
+#pragma unroll
+    for (int z = 0; z < EPT; ++z) {
+        const int idx = tid + z * NT;
+        es[z] = idx < NN ? idx / N : 0;
+        ek[z] = idx < NN ? idx % N : 0;
+        ch[z] = idx < NN ? chi[idx] : 0.f;
+        // the step to the final state: a_{L-1}[s] chi[s][final] / P
+        cs[z] = idx < NN && ek[z] == A.fin ? __fmul_rn(al[(int64_t)(L - 1) * N + es[z]] * ch[z], s_f[0]) : 0.f;
+        cc[z] = 0.f;
     }
-    float mx = 0.f;
-    for (int s = tid; s < N; s += NT) {
-        vw[s] = chi[s * NP + final_state];
-        mx = fmaxf(mx, vw[s]);
-    }
-    mx = block_max(mx, redf);
-    int eb = mx > 0.f ? exp2_of(mx) : 0;
-    for (int s = tid; s < N; s += NT) va[s] = mx > 0.f ? ldexpf(vw[s], -eb) : 0.f;
-    int cumb = mx > 0.f ? eb : EXPN;
-    __syncthreads();
-    if (post) {
-        const float f = (float)exp2((double)ae[L - 1] + (double)cumb - lp2);
-        for (int k = tid; k < N; k += NT)
-            post[(m.off + L - 1) * N + k] = al[(int64_t)(L - 1) * N + k] * va[k] * f;
-    }
-    for (int l = L - 2; l >= -1; --l) {
-        // w[k] = e_{l+1}[k] b_{l+1}[k]
-        for (int k = tid; k < N; k += NT) vw[k] = em[(int64_t)(l + 1) * N + k] * va[k];
+    for (int top = L - 1; top >= 0; top -= TILE) {   // columns top, top - 1, ...
+        const int n = min(TILE, top + 1);
         __syncthreads();
-        if (l < 0) break;   // vw now holds e_0 .* b_0 for the initial counts
-        // interior counts: n[s][k] += a_l[s] chi[s][k] w[k] 2^(A_l + B_{l+1} - log2 P)
-        const float f = (float)exp2((double)ae[l] + (double)cumb - lp2);
-        const float *alr = al + (int64_t)l * N;
-        for (int idx = tid; idx < N * N; idx += NT) {
-            const int s = idx / N, k = idx % N;
-            const float v = alr[s] * chi[s * NP + k] * vw[k];
-            if (v != 0.f) add(idx, v * f);
+        if (tid < 2 * TILE) {
+            const int i = tid % TILE, l = top - i, ln = tid < TILE ? l + 1 : l;
+            if (i < n) scale[tid / TILE][i] = ln < L ? (float)exp2((double)ae[l] + (double)bx[ln] - lp2) : 0.f;
         }
-        // b_l[s] = sum_k chi[s][k] w[k]
-        float mxb = 0.f;
-        float bnew[(MAXN + NT - 1) / NT];
-        for (int s = tid, q = 0; s < N; s += NT, ++q) {
-            float acc = 0.f;
-            for (int k = 0; k < N; ++k) acc = fmaf(chi[s * NP + k], vw[k], acc);
-            bnew[q] = acc;
-            mxb = fmaxf(mxb, acc);
+        for (int q = tid; q < n * N; q += NT) {
+            const int i = q / N, k = q - i * N, l = top - i;
+            ta[q] = al[(int64_t)l * N + k];
+            tw[q] = l + 1 < L ? em[(int64_t)(l + 1) * N + k] * be[(int64_t)(l + 1) * N + k] : 0.f;
         }
-        mxb = block_max(mxb, redf);
-        eb = mxb > 0.f ? exp2_of(mxb) : 0;
-        for (int s = tid, q = 0; s < N; s += NT, ++q) va[s] = mxb > 0.f ? ldexpf(bnew[q], -eb) : 0.f;
-        cumb = (mxb > 0.f && cumb > EXPN) ? cumb + eb : EXPN;
         __syncthreads();
-        if (post) {
-            const float g = (float)exp2((double)ae[l] + (double)cumb - lp2);
-            for (int k = tid; k < N; k += NT) post[(m.off + l) * N + k] = alr[k] * va[k] * g;
+        if (A.post)
+            for (int q = tid; q < n * N; q += NT) {
+                const int i = q / N, k = q - i * N, l = top - i;
+                A.post[(m.off + l) * N + k] = ta[q] * be[(int64_t)l * N + k] * scale[1][i];
+            }
+        // n[s][k] += a_l[s] chi[s][k] w_{l+1}[k] 2^(A_l + B_{l+1} - log2 P)
+        for (int i = top == L - 1 ? 1 : 0; i < n; ++i) {
+            const float f = scale[0][i];
+            const float *a = ta + i * N, *w = tw + i * N;
+#pragma unroll
+            for (int z = 0; z < EPT; ++z) {
+                const float v = a[es[z]] * ch[z] * w[ek[z]];
+                if (v != 0.f) add(cs[z], cc[z], v, f);
+            }
         }
     }
-    // initial: n[init][k] += chi[init][k] e_0[k] b_0[k] / P  (vw = e_0 .* b_0 at exponent cumb)
-    {
-        const float f = (float)exp2((double)cumb - lp2);
-        for (int k = tid; k < N; k += NT) add(init_state * N + k, chi[init_state * NP + k] * vw[k] * f);
+#pragma unroll
+    for (int z = 0; z < EPT; ++z) {
+        const int idx = tid + z * NT;
+        if (idx >= NN) break;
+        // the step from the initial state: chi[init][k] e_0[k] b_0[k] / P
+        if (es[z] == A.init) add(cs[z], cc[z], ch[z] * (em[ek[z]] * be[ek[z]]), s_f[1]);
+        nt[idx] = (double)cs[z] - (double)cc[z];
     }
-    __syncthreads();
-    for (int idx = tid; idx < N * N; idx += NT) nt[idx] = (double)cs[idx] - (double)cc[idx];
+}
+
+template <int NB, int NR, int NT, int EPT>
+cudaError_t launch(const Args &a, int P, cudaStream_t st) {
+    const size_t smem = sizeof(float) * ((size_t)a.N * a.N + 2 * TILE * a.N);
+    fb1d_kernel<NB, NR, NT, EPT><<<P, NT, smem, st>>>(a);
+    return cudaGetLastError();
 }
 
 // Per-column emissions of an alignment: column l of type c (1 M, 2 I, 3 D)
@@ -216,35 +316,36 @@ struct EmitDesc {
     int8_t group[MAXN];
 };
 
+// One warp per column, a lane per state; blockIdx.y takes columns of its own.
 __global__ void __launch_bounds__(256)
 emit1d_kernel(const __grid_constant__ EmitDesc ed, const Meta *__restrict__ meta, const uint8_t *__restrict__ cols,
               const uint8_t *__restrict__ anc, const uint8_t *__restrict__ desc, const float *__restrict__ tM,
               const float *__restrict__ tI, const float *__restrict__ tD, int per_pair, int G,
               float *__restrict__ emit, int32_t *__restrict__ status) {
-    const int p = blockIdx.x;
+    const int p = blockIdx.x, lane = threadIdx.x & 31;
     const Meta m = meta[p];
     const int N = ed.N;
     const float *M_ = tM + (per_pair ? (int64_t)p * G * 441 : 0);
     const float *I_ = tI + (per_pair ? (int64_t)p * G * 21 : 0);
     const float *D_ = tD + (per_pair ? (int64_t)p * G * 21 : 0);
-    for (int64_t idx = threadIdx.x; idx < (int64_t)m.L * N; idx += blockDim.x) {
-        const int64_t l = idx / N;
-        const int s = (int)(idx % N);
+    for (int l = blockIdx.y * 8 + (threadIdx.x >> 5); l < m.L; l += gridDim.y * 8) {
         const int c = cols[m.off + l];
         int a = anc[m.off + l], b = desc[m.off + l];
         if (a > 20 || b > 20) {
-            atomicOr(status + p, PHMM_ST_BAD_RESIDUE);
+            if (lane == 0) atomicOr(status + p, PHMM_ST_BAD_RESIDUE);
             a = a > 20 ? 20 : a;
             b = b > 20 ? 20 : b;
         }
-        float v = 0.f;
-        if (c == ed.type[s]) {
-            const int g = ed.group[s];
-            if (c == 1) v = M_[g * 441 + a * 21 + b];
-            else if (c == 2) v = I_[g * 21 + b];
-            else if (c == 3) v = D_[g * 21 + a];
+        for (int s = lane; s < N; s += 32) {
+            float v = 0.f;
+            if (c == ed.type[s]) {
+                const int g = ed.group[s];
+                if (c == 1) v = M_[g * 441 + a * 21 + b];
+                else if (c == 2) v = I_[g * 21 + b];
+                else if (c == 3) v = D_[g * 21 + a];
+            }
+            emit[(m.off + l) * N + s] = v;
         }
-        emit[(m.off + l) * N + s] = v;
     }
 }
 
@@ -266,8 +367,8 @@ static int fb1_layout(int P, const int32_t *L_host, const int64_t *off_host, int
     }
     const size_t o_meta = 0;
     *o_alpha = fb1_align(o_meta + sizeof(fb1::Meta) * (size_t)P);
-    *o_aexp = fb1_align(*o_alpha + sizeof(float) * cols * N);
-    *total = fb1_align(*o_aexp + sizeof(int) * cols);
+    *o_aexp = fb1_align(*o_alpha + 2 * sizeof(float) * cols * N);   // alpha, then beta
+    *total = fb1_align(*o_aexp + 2 * sizeof(int) * cols);
     *cols_out = cols;
     return PHMM_OK;
 }
@@ -308,14 +409,28 @@ extern "C" int phmm_fb1d(const phmm_fb1d_batch *b, void *workspace, size_t works
     cudaError_t e = cudaMemcpyAsync(ws, meta.data(), sizeof(Meta) * P, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(status_out, 0, sizeof(int32_t) * P, st);
     if (e != cudaSuccess) return fb1_fail(PHMM_E_CUDA, cudaGetErrorString(e));
-    const int NP = N | 1;
-    const size_t smem = sizeof(float) * ((size_t)N * NP + 2 * MAXN + 2 * MAXN * MAXN);
-    e = cudaFuncSetAttribute(fb1d_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return fb1_fail(PHMM_E_CUDA, cudaGetErrorString(e));
-    fb1d_kernel<<<P, NT, smem, st>>>((const Meta *)ws, N, b->chi, b->chi_per_pair, b->emit, b->init_state,
-                                    b->final_state, (float *)(ws + oa), (int *)(ws + oe), ll_out, n_trans,
-                                    posteriors, status_out);
-    e = cudaGetLastError();
+    Args a;
+    a.meta = (const Meta *)ws;
+    a.N = N;
+    a.chi_per_pair = b->chi_per_pair;
+    a.init = b->init_state;
+    a.fin = b->final_state;
+    a.chi = b->chi;
+    a.emit = b->emit;
+    a.alpha = (float *)(ws + oa);
+    a.beta = a.alpha + cols * N;
+    a.aexp = (int *)(ws + oe);
+    a.bexp = a.aexp + cols;
+    a.ll = ll_out;
+    a.n = n_trans;
+    a.post = posteriors;
+    a.status = status_out;
+    // one state per recursion lane up to 32 states, two above; the bounds keep the padding of the products small
+    if (N <= 8) e = launch<8, 1, 64, 1>(a, P, st);
+    else if (N <= 20) e = launch<20, 1, 256, 2>(a, P, st);
+    else if (N <= 32) e = launch<32, 1, 256, 4>(a, P, st);
+    else if (N <= 44) e = launch<44, 2, 256, 8>(a, P, st);
+    else e = launch<64, 2, 256, 16>(a, P, st);
     if (e != cudaSuccess) return fb1_fail(PHMM_E_CUDA, cudaGetErrorString(e));
     return PHMM_OK;
 }
@@ -355,7 +470,9 @@ extern "C" int phmm_fb1d_emissions(const phmm_model_desc *model, int32_t n_pairs
     cudaError_t e = cudaMemcpyAsync(workspace, meta.data(), sizeof(Meta) * n_pairs, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(status_out, 0, sizeof(int32_t) * n_pairs, st);
     if (e != cudaSuccess) return fb1_fail(PHMM_E_CUDA, cudaGetErrorString(e));
-    emit1d_kernel<<<n_pairs, 256, 0, st>>>(ed, (const Meta *)workspace, cols, anc, desc, emit_M, emit_I, emit_D,
+    int most = 1;
+    for (const Meta &m : meta) most = std::max(most, (int)m.L);
+    emit1d_kernel<<<dim3(n_pairs, std::min(16, (most + 31) / 32)), 256, 0, st>>>(ed, (const Meta *)workspace, cols, anc, desc, emit_M, emit_I, emit_D,
                                           emit_per_pair, G, emit, status_out);
     e = cudaGetLastError();
     if (e != cudaSuccess) return fb1_fail(PHMM_E_CUDA, cudaGetErrorString(e));
