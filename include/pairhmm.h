@@ -460,6 +460,16 @@ typedef struct phmm_tkf92_params {
 int phmm_tkf92_tables(const phmm_tkf92_params *prm, int32_t n_pairs, const double *t, float *chi,
                       float *emit_M, float *emit_I, float *emit_D, double *sub, void *stream);
 
+/* Device epilogue of the batched TKF92 E-step (train/tkf92_svi_bw.py:75-171,
+ * 263-334; core/bdi.py:682-780) from its expected transitions n_trans [P][5][5]
+ * and the pairs' times t [P] (device float64): stats [7][P] (device float64) holds
+ * E[B], E[D], E[S] (floored at 0), the log kappa and log(1 - kappa) coefficients,
+ * the fragment extensions and the body rows' remaining total; resolved (nullable)
+ * [P][5][5] the counts without the extensions.  Rates closer than 1e-10 (relative)
+ * are refused: E[S] then needs its limit form. */
+int phmm_tkf92_bdi(double ins_rate, double del_rate, double ext, int32_t n_pairs, const double *t,
+                   const double *n_trans, double *stats, double *resolved, void *stream);
+
 /* Device epilogue of the MixDom2 E-step: the per-class sufficient statistics
  * of train/likelihood.py:279-344 from phmm_estep's per-group character
  * counts (cnt_M [P][KF][21][21], cnt_I / cnt_D [P][KF][21]) and the

@@ -23,7 +23,7 @@ EXPORTS = ('phmm_plan_create', 'phmm_plan_destroy', 'phmm_forward', 'phmm_estep'
            'phmm_set_variant', 'phmm_set_spin_limit', 'phmm_set_tuning', 'phmm_get_tuning',
            'phmm_last_variant', 'phmm_last_launch_count',
            'phmm_last_error', 'phmm_version', 'phmm_mixdom2_class_subs_count', 'phmm_mixdom2_tables',
-           'phmm_mixdom2_class_counts', 'phmm_tkf92_tables', 'phmm_mixdom2_chi',
+           'phmm_mixdom2_class_counts', 'phmm_tkf92_tables', 'phmm_tkf92_bdi', 'phmm_mixdom2_chi',
            'phmm_mixdom2_chi_vjp_dirs', 'phmm_mixdom2_chi_vjp', 'phmm_fb1d_workspace_bytes', 'phmm_fb1d',
            'phmm_fb1d_emissions', 'phmm_viterbi_workspace_bytes', 'phmm_viterbi', 'phmm_holmes_rubin',
            'phmm_sample_workspace_bytes', 'phmm_sample_paths', 'phmm_pairs_count', 'phmm_pairs_decode',
@@ -159,6 +159,8 @@ def load(path=None):
     lib.phmm_mixdom2_chi_vjp.restype = ctypes.c_int
     lib.phmm_tkf92_tables.argtypes = [ctypes.POINTER(Tkf92Params), ctypes.c_int32] + [vp] * 7
     lib.phmm_tkf92_tables.restype = ctypes.c_int
+    lib.phmm_tkf92_bdi.argtypes = [ctypes.c_double] * 3 + [ctypes.c_int32] + [vp] * 5
+    lib.phmm_tkf92_bdi.restype = ctypes.c_int
     lib.phmm_fb1d_workspace_bytes.argtypes = [ctypes.POINTER(Fb1dBatch), ctypes.POINTER(ctypes.c_size_t)]
     lib.phmm_fb1d_workspace_bytes.restype = ctypes.c_int
     lib.phmm_fb1d.argtypes = [ctypes.POINTER(Fb1dBatch), vp, ctypes.c_size_t, vp, vp, vp, vp, vp]
@@ -839,6 +841,19 @@ def tkf92_tables(ins_rate, del_rate, ext, Q, pi, ts, device='cuda', stream=None)
     times ts: (chi [P,5,5] f32, EM [P,1,21,21] f32, EI [P,1,21] f32, ED
     [P,1,21] f32, sub [P,20,20] f64) device tensors."""
     return Tkf92Prologue(ins_rate, del_rate, ext, Q, pi)(ts, device=device, stream=stream)
+
+
+def tkf92_bdi(n_trans, ins_rate, del_rate, t, ext, stream=None):
+    """phmm_tkf92_bdi: (stats [7, P], resolved [P, 5, 5]) float64 device tensors
+    for device counts n_trans [P, 5, 5] and times t [P] (float64, contiguous)."""
+    lib = load()
+    P, dev = n_trans.shape[0], n_trans.device
+    stats = torch.empty(7, P, dtype=torch.float64, device=dev)
+    res = torch.empty(P, 5, 5, dtype=torch.float64, device=dev)
+    s = stream if stream is not None else torch.cuda.current_stream(dev)
+    _check(lib.phmm_tkf92_bdi(float(ins_rate), float(del_rate), float(ext), P, _ptr(t), _ptr(n_trans), _ptr(stats),
+                              _ptr(res), ctypes.c_void_p(s.cuda_stream)), 'phmm_tkf92_bdi')
+    return stats, res
 
 
 def sample_paths(state_types, groups, G, xs, ys, log_chi, log_M, log_I, log_D, n_samples, seed,

@@ -12,7 +12,9 @@ Restates, batched over pairs in torch float64:
     automatic differentiation, the conservation term, and either the general
     formula or, for |1 - kappa| < 1e-10, the L'Hopital limit E[S] = f'(mu).
 Negative values from cancellation are clamped at zero as the reference does
-(train/tkf92_svi_bw.py:318-320).
+(train/tkf92_svi_bw.py:318-320).  Device counts of the TKF92 E-step take one
+kernel for all of it (phmm_tkf92_bdi); the tensor form here serves host counts,
+equal rates, a separate T and differentiated counts.
 """
 from __future__ import annotations
 
@@ -128,6 +130,16 @@ def kappa_coefficients(res):
 
 def tkf92_bdi_epilogue(n_chi, ins_rate, del_rate, t, ext, T=None):
     """The dict of estep_batch_tkf92 beyond log_p (train/tkf92_svi_bw.py:263-334)."""
+    lam, mu, x = float(ins_rate), float(del_rate), float(ext)
+    if (T is None and isinstance(n_chi, torch.Tensor) and n_chi.is_cuda and not n_chi.requires_grad and lam > 0.0
+            and mu > 0.0 and abs(1.0 - lam / mu) >= ES_LHOPITAL_THRESHOLD and 0.0 <= x < 1.0):
+        from . import _lib
+        n = pm._t(n_chi).contiguous()
+        tt = pm._t(t, device=n.device).reshape(-1)
+        if n.dim() == 3 and tt.numel() == n.shape[0]:
+            stats, res = _lib.tkf92_bdi(n, lam, mu, tt.contiguous(), x)
+            keys = ('B', 'D', 'S', 'L', 'M', 'ext_count', 'notext_count')
+            return {**dict(zip(keys, stats.unbind(0))), 'T': tt, 'n_trans_resolved': res}
     res, ext_count, notext = tkf92_resolve(n_chi, ins_rate, del_rate, t, ext)
     L, Mc = kappa_coefficients(res)
     tt = pm._t(t, device=res.device).reshape(-1)
