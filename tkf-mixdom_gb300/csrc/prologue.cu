@@ -13,11 +13,7 @@
 //                  right-hand sides), T_exit_k, the effective 5x5 T, and the
 //                  N x N collapsed matrix written as float32;
 //   expm_kernel    one CTA per (pair, class): Q_c from (S_exch, pi), then
-//                  exp(t Q_c) by scaling and squaring with the degree-13 Pade
-//                  approximant of Higham, "The scaling and squaring method
-//                  for the matrix exponential revisited", SIAM J. Matrix
-//                  Anal. Appl. 26 (2005), Algorithm 2.3 (the method
-//                  jax.scipy.linalg.expm implements), float64;
+//                  exp(t Q_c) by a scaled Taylor polynomial, float64;
 //   tables_kernel  one CTA per pair: EM[g][a][b] = sum_c w[g][c]
 //                  max(pi_c[a],1e-30) max(P_c[a][b],1e-30), EI = ED =
 //                  sum_c w[g][c] max(pi_c[a],1e-30), wildcard factor 1.
@@ -433,20 +429,36 @@ chi_vjp_kernel(const __grid_constant__ Packed prm, const double *__restrict__ ts
     }
 }
 
-// ---------------------------------------------------------------- expm (Pade 13)
-// b_j of the [13/13] Pade approximant of exp (Higham 2005, eq. 2.1 / Table 2.3)
-__device__ __constant__ double PADE13[14] = {
-    64764752532480000.0, 32382376266240000.0, 7771770303897600.0, 1187353796428800.0,
-    129060195264000.0, 10559470521600.0, 670442572800.0, 33522128640.0,
-    1323241920.0, 40840800.0, 960960.0, 16380.0, 182.0, 1.0};
-// theta_13 of the same paper: the 1-norm up to which degree 13 needs no scaling
-constexpr double THETA13 = 5.371920351148152;
+// ---------------------------------------------------------------- expm
+// exp(X) by its Taylor polynomial T_m on X / 2^s, m = 8, 12 or 16, evaluated in
+// blocks of four powers (Paterson and Stockmeyer, "On the number of nonscalar
+// multiplications necessary to evaluate polynomials", SIAM J. Comput. 2 (1973)):
+// X^2, X^3, X^4, then m / 4 - 1 products by X^4, and s squarings.  Up to the
+// 1-norm bounds below the first term left out, also entry by entry against X,
+// is under half an ulp (theta^m (m + 1) / (m + 1)! < 2^-53).
+// FP64 products bound it: a 20 x 20 product is 8000 multiply-adds on an SM's two
+// FP64 lanes, 2 us.  Six products and s squarings of one CTA replace the
+// degree-13 Pade form's six, its 20 x 40 elimination with a barrier chain per
+// column, and squarings: 71 -> 32 us for 4 to 64 matrices at times up to 2 (one an SM), 100 -> 61 us for 256.
+constexpr double THETA8 = 0.06, THETA12 = 0.3, THETA16 = 0.7;
+__device__ __constant__ double INV_FACT[17] = {
+    1.0, 1.0, 1.0 / 2, 1.0 / 6, 1.0 / 24, 1.0 / 120, 1.0 / 720, 1.0 / 5040, 1.0 / 40320, 1.0 / 362880, 1.0 / 3628800,
+    1.0 / 39916800, 1.0 / 479001600, 1.0 / 6227020800.0, 1.0 / 87178291200.0, 1.0 / 1307674368000.0,
+    1.0 / 20922789888000.0};
 
-__device__ void mm(double *C, const double *A, const double *B, int n) {
-    for (int idx = threadIdx.x; idx < n * n; idx += blockDim.x) {
-        const int i = idx / n, j = idx % n;
-        double s = 0.0;
-        for (int k = 0; k < n; ++k) s += A[i * n + k] * B[k * n + j];
+// C = A B + sum_i c[i] X^i (i = 0..3 over the identity, X, X2, X3; c null: C = A B)
+__device__ __forceinline__ void mm20(double *C, const double *A, const double *B, const double *c = nullptr,
+                                     const double *X = nullptr, const double *X2 = nullptr, const double *X3 = nullptr) {
+    for (int idx = threadIdx.x; idx < NA * NA; idx += blockDim.x) {
+        const int i = idx / NA, j = idx % NA;
+        double s = 0.0, u = 0.0;
+#pragma unroll
+        for (int k = 0; k < NA; k += 2) {
+            s += A[i * NA + k] * B[k * NA + j];
+            u += A[i * NA + k + 1] * B[(k + 1) * NA + j];
+        }
+        s += u;
+        if (c) s += (i == j ? c[0] : 0.0) + c[1] * X[idx] + c[2] * X2[idx] + c[3] * X3[idx];
         C[idx] = s;
     }
     __syncthreads();
@@ -454,10 +466,9 @@ __device__ void mm(double *C, const double *A, const double *B, int n) {
 
 __device__ __forceinline__ void expm_kernel_body(const Packed &prm, const double *__restrict__ ts, double *__restrict__ csubs) {
     constexpr int n = NA, nn = NA * NA;
-    __shared__ double X[nn], A2[nn], A4[nn], A6[nn], W1[nn], W2[nn], U[nn], V[nn];
-    __shared__ double aug[n * 2 * n];
+    __shared__ double X[nn], X2[nn], X3[nn], X4[nn], W1[nn], W2[nn];
     __shared__ double colsum[n];
-    __shared__ int piv_row, n_sq;
+    __shared__ int n_sq, n_deg;
     const int p = blockIdx.x / prm.C, c = blockIdx.x % prm.C, tid = threadIdx.x;
     const double t = ts[p];
     const double *Sx = prm.v + prm.o_S + (size_t)c * nn, *pi = prm.v + prm.o_pis + c * n;
@@ -478,91 +489,43 @@ __device__ __forceinline__ void expm_kernel_body(const Packed &prm, const double
         }
     }
     __syncthreads();
-    for (int idx = tid; idx < nn; idx += blockDim.x) X[idx] *= t;
-    __syncthreads();
     if (tid < n) {
         double s = 0.0;
         for (int a = 0; a < n; ++a) s += fabs(X[a * n + tid]);
-        colsum[tid] = s;
+        colsum[tid] = s * fabs(t);
     }
     __syncthreads();
     if (tid == 0) {
         double nrm = 0.0;
         for (int b = 0; b < n; ++b) nrm = fmax(nrm, colsum[b]);
         int s = 0;
-        if (nrm > THETA13) s = (int)ceil(log2(nrm / THETA13));
+        if (nrm > THETA16) s = (int)ceil(log2(nrm / THETA16));
         n_sq = s < 0 ? 0 : (s > 60 ? 60 : s);
+        n_deg = nrm <= THETA8 ? 8 : nrm <= THETA12 ? 12 : 16;
     }
     __syncthreads();
-    const int s = n_sq;
-    for (int idx = tid; idx < nn; idx += blockDim.x) X[idx] = ldexp(X[idx], -s);
+    const int s = n_sq, m = n_deg;
+    for (int idx = tid; idx < nn; idx += blockDim.x) X[idx] = ldexp(X[idx] * t, -s);
     __syncthreads();
-    mm(A2, X, X, n);
-    mm(A4, A2, A2, n);
-    mm(A6, A4, A2, n);
-    const double *b = PADE13;
-    // W1 = b13 A6 + b11 A4 + b9 A2;  W2 = b12 A6 + b10 A4 + b8 A2
+    mm20(X2, X, X);
+    mm20(X3, X2, X);
+    mm20(X4, X2, X2);
+    // T_m = (.. (X^4 / m! + B_{m/4-1}) X^4 + ..) X^4 + B_0, B_j = sum_{i<4} X^i / (4 j + i)!
     for (int idx = tid; idx < nn; idx += blockDim.x) {
-        W1[idx] = b[13] * A6[idx] + b[11] * A4[idx] + b[9] * A2[idx];
-        W2[idx] = b[12] * A6[idx] + b[10] * A4[idx] + b[8] * A2[idx];
+        const double *f = INV_FACT + m - 4;
+        W1[idx] = (idx / n == idx % n ? f[0] : 0.0) + f[1] * X[idx] + f[2] * X2[idx] + f[3] * X3[idx] + f[4] * X4[idx];
     }
     __syncthreads();
-    mm(U, A6, W1, n);   // A6 W1
-    mm(V, A6, W2, n);   // A6 W2
-    for (int idx = tid; idx < nn; idx += blockDim.x) {
-        const double id = (idx / n == idx % n) ? 1.0 : 0.0;
-        W1[idx] = U[idx] + b[7] * A6[idx] + b[5] * A4[idx] + b[3] * A2[idx] + b[1] * id;
-        V[idx] = V[idx] + b[6] * A6[idx] + b[4] * A4[idx] + b[2] * A2[idx] + b[0] * id;
-    }
-    __syncthreads();
-    mm(U, X, W1, n);    // U = X (A6 W1 + ...)
-    // solve (V - U) R = (V + U)
-    for (int idx = tid; idx < nn; idx += blockDim.x) {
-        const int i = idx / n, j = idx % n;
-        aug[i * 2 * n + j] = V[idx] - U[idx];
-        aug[i * 2 * n + n + j] = V[idx] + U[idx];
-    }
-    __syncthreads();
-    const int w = 2 * n;
-    for (int cc = 0; cc < n; ++cc) {
-        if (tid == 0) {
-            int best = cc;
-            double bv = fabs(aug[cc * w + cc]);
-            for (int r = cc + 1; r < n; ++r) {
-                const double v = fabs(aug[r * w + cc]);
-                if (v > bv) { bv = v; best = r; }
-            }
-            piv_row = best;
-        }
-        __syncthreads();
-        const int pr = piv_row;
-        if (pr != cc)
-            for (int j = tid; j < w; j += blockDim.x) {
-                const double a = aug[cc * w + j];
-                aug[cc * w + j] = aug[pr * w + j];
-                aug[pr * w + j] = a;
-            }
-        __syncthreads();
-        const double inv = 1.0 / aug[cc * w + cc];
-        __syncthreads();
-        for (int j = tid; j < w; j += blockDim.x) aug[cc * w + j] *= inv;
-        __syncthreads();
-        for (int idx = tid; idx < n * w; idx += blockDim.x) {
-            const int r = idx / w, j = idx % w;
-            if (r == cc || j == cc) continue;
-            aug[idx] -= aug[r * w + cc] * aug[cc * w + j];
-        }
-        __syncthreads();
-        for (int r = tid; r < n; r += blockDim.x)
-            if (r != cc) aug[r * w + cc] = 0.0;
-        __syncthreads();
-    }
-    for (int idx = tid; idx < nn; idx += blockDim.x) W1[idx] = aug[(idx / n) * w + n + idx % n];
-    __syncthreads();
-    // undo the scaling: square s times
     double *cur = W1, *nxt = W2;
+    for (int j = m / 4 - 2; j >= 0; --j) {
+        mm20(nxt, cur, X4, INV_FACT + 4 * j, X, X2, X3);
+        double *tmp = cur;
+        cur = nxt;
+        nxt = tmp;
+    }
+    // undo the scaling: square s times
     for (int k = 0; k < s; ++k) {
-        mm(nxt, cur, cur, n);
+        mm20(nxt, cur, cur);
         double *tmp = cur;
         cur = nxt;
         nxt = tmp;
@@ -629,68 +592,83 @@ tables_kernel_dp(const Packed *__restrict__ prm, const double *__restrict__ csub
 // the reference's clamped gather for the wildcard) and w[g][c] = classdist,
 //   match[c][a][b] = sum_g cM[g][a][b] w[g][c] f_c[a][b] / sum_c' w[g][c'] f_c'[a][b]
 // (insert / delete alike with pi_c[a']), classdist[g][c] = the sum over all
-// 21 x 21 (and 21) characters of the same terms.  One CTA per pair.
-constexpr int CS_MAXC = 8;
+// 21 x 21 (and 21) characters of the same terms.
+// The characters are 483 columns (441 match, 21 insert, 21 delete) taken 32 at a
+// time, one per lane, the groups split over the warps; the columns spread over
+// gridDim.y CTAs, which add their shares of classdist (zeroed before) when there
+// is more than one.  FP64 bounds it (a division per group and column, none with
+// one class): one CTA per pair, a division per class and an atomic per term, took
+// 1.19 ms for 4 pairs of 32 groups and 4 classes, now 24 us; 200 pairs of 3 groups
+// and one class 98 us, now 33 us.
+constexpr int CS_MAXC = 8, CS_COLS = 441 + 42, CS_CHUNKS = (CS_COLS + 31) / 32;
 
 __device__ __forceinline__ void class_split_kernel_body(const Packed &prm, const double *__restrict__ csubs,
                    const double *__restrict__ cM, const double *__restrict__ cI, const double *__restrict__ cD,
                    double *__restrict__ match, double *__restrict__ ins, double *__restrict__ del,
                    double *__restrict__ cdist) {
-    extern __shared__ double cs_acc[];   // [G][C] classdist partial sums
-    const int p = blockIdx.x, tid = threadIdx.x;
+    extern __shared__ double cs_acc[];   // [G][C] classdist sums, then [warps][C][32] class sums of a chunk's columns
+    const int p = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, NW = blockDim.x >> 5;
     const int C = prm.C, G = prm.K * prm.F;
     const double *cd = prm.v + prm.o_cd, *pis = prm.v + prm.o_pis;
     const double *Pp = csubs + (size_t)p * C * NA * NA;
+    double *part = cs_acc + G * C;
     for (int i = tid; i < G * C; i += blockDim.x) cs_acc[i] = 0.0;
     __syncthreads();
-    double loc[CS_MAXC];
-    // match-type cells
-    for (int ab = tid; ab < 441; ab += blockDim.x) {
-        const int a = ab / 21, b = ab % 21;
-        const int ac = a < NA ? a : NA - 1, bc = b < NA ? b : NA - 1;
+    for (int chunk = blockIdx.y; chunk < CS_CHUNKS; chunk += gridDim.y) {
+        const int x = chunk * 32 + lane;
+        const bool in = x < CS_COLS, is_match = x < 441;
+        const int one = (x - 441) % 21;   // the character of an insert / delete column
+        const int a = is_match ? x / 21 : one, b = is_match ? x % 21 : 0;
+        const int ac = min(a, NA - 1), bc = min(b, NA - 1);
+        const double *cnt = is_match ? cM + (size_t)p * G * 441 + x
+                                     : (x < 462 ? cI : cD) + (size_t)p * G * 21 + (in ? one : 0);
+        const int stride = is_match ? 441 : 21;
         double f[CS_MAXC], acc[CS_MAXC];
-        for (int c = 0; c < C; ++c) {
-            f[c] = pis[c * NA + ac] * Pp[(c * NA + ac) * NA + bc];
+#pragma unroll
+        for (int c = 0; c < CS_MAXC; ++c) {
+            if (c >= C) break;
+            f[c] = in ? (is_match ? pis[c * NA + ac] * Pp[(c * NA + ac) * NA + bc] : pis[c * NA + ac]) : 0.0;
             acc[c] = 0.0;
         }
-        for (int g = 0; g < G; ++g) {
+        for (int g = warp; g < G; g += NW) {
+            const double n = in ? cnt[(size_t)g * stride] : 0.0;
             double den = 0.0;
-            for (int c = 0; c < C; ++c) den += cd[g * C + c] * f[c];
-            const double n = cM[((size_t)p * G + g) * 441 + ab];
-            for (int c = 0; c < C; ++c) {
-                const double wgc = n * (cd[g * C + c] * f[c] / (den + 1e-300));
-                acc[c] += wgc;
-                loc[c] = wgc;
+#pragma unroll
+            for (int c = 0; c < CS_MAXC; ++c) {
+                if (c >= C) break;
+                den += cd[g * C + c] * f[c];
             }
-            for (int c = 0; c < C; ++c) atomicAdd(&cs_acc[g * C + c], loc[c]);
-        }
-        if (a < NA && b < NA)
-            for (int c = 0; c < C; ++c) match[(((size_t)p * C + c) * NA + a) * NA + b] = acc[c];
-    }
-    // insert / delete cells: the same posterior over pi_c
-    for (int ia = tid; ia < 2 * 21; ia += blockDim.x) {
-        const bool is_ins = ia < 21;
-        const int a = ia % 21, ac = a < NA ? a : NA - 1;
-        const double *cnt = is_ins ? cI : cD;
-        double acc[CS_MAXC];
-        for (int c = 0; c < C; ++c) acc[c] = 0.0;
-        for (int g = 0; g < G; ++g) {
-            double den = 0.0;
-            for (int c = 0; c < C; ++c) den += cd[g * C + c] * pis[c * NA + ac];
-            const double n = cnt[((size_t)p * G + g) * 21 + a];
-            for (int c = 0; c < C; ++c) {
-                const double wgc = n * (cd[g * C + c] * pis[c * NA + ac] / (den + 1e-300));
-                acc[c] += wgc;
-                atomicAdd(&cs_acc[g * C + c], wgc);
+            // one class has all of the column (x / (x + 1e-300) is 1 in float64)
+            const bool whole = C == 1 && den > 1e-280;
+            const double q = whole ? n : den > 0.0 ? n / (den + 1e-300) : 0.0;
+#pragma unroll
+            for (int c = 0; c < CS_MAXC; ++c) {
+                if (c >= C) break;
+                double w = whole ? n : (cd[g * C + c] * f[c]) * q;
+                acc[c] += w;
+                for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+                if (lane == 0) cs_acc[g * C + c] += w;   // the group is this warp's
             }
         }
-        if (a < NA) {
-            double *out = is_ins ? ins : del;
-            for (int c = 0; c < C; ++c) out[((size_t)p * C + c) * NA + a] = acc[c];
+#pragma unroll
+        for (int c = 0; c < CS_MAXC; ++c) {
+            if (c >= C) break;
+            part[(warp * C + c) * 32 + lane] = acc[c];
         }
+        __syncthreads();
+        if (in && a < NA && b < NA)
+            for (int c = warp; c < C; c += NW) {
+                double v = 0.0;
+                for (int w = 0; w < min(NW, G); ++w) v += part[(w * C + c) * 32 + lane];
+                if (is_match) match[(((size_t)p * C + c) * NA + a) * NA + b] = v;
+                else (x < 462 ? ins : del)[((size_t)p * C + c) * NA + a] = v;
+            }
+        __syncthreads();
     }
-    __syncthreads();
-    for (int i = tid; i < G * C; i += blockDim.x) cdist[(size_t)p * G * C + i] = cs_acc[i];
+    for (int i = tid; i < G * C; i += blockDim.x) {
+        if (gridDim.y == 1) cdist[(size_t)p * G * C + i] = cs_acc[i];
+        else atomicAdd(&cdist[(size_t)p * G * C + i], cs_acc[i]);
+    }
 }
 
 __global__ void __launch_bounds__(THREADS)
@@ -703,6 +681,19 @@ class_split_kernel(const __grid_constant__ Packed prm, const double *__restrict_
 __global__ void __launch_bounds__(THREADS)
 class_split_kernel_dp(const Packed *__restrict__ prm, const double *__restrict__ csubs, const double *__restrict__ cM, const double *__restrict__ cI, const double *__restrict__ cD, double *__restrict__ match, double *__restrict__ ins, double *__restrict__ del, double *__restrict__ cdist) {
     class_split_kernel_body(*prm, csubs, cM, cI, cD, match, ins, del, cdist);
+}
+
+// Launch shape of the class split: warps by groups (a warp takes whole groups), and
+// as many column CTAs per pair as bring the grid to about two per SM.
+struct SplitShape {
+    int threads, parts;
+    size_t smem;
+};
+inline SplitShape split_shape(int P, int G, int C) {
+    const int warps = G < THREADS / 32 ? G : THREADS / 32;
+    int parts = 1;
+    while (parts < CS_CHUNKS && (int64_t)P * parts * 2 <= 304) parts *= 2;
+    return {warps * 32, parts, sizeof(double) * ((size_t)G * C + (size_t)warps * C * 32)};
 }
 
 // ---------------------------------------------------------------- TKF92 prologue
@@ -943,10 +934,14 @@ extern "C" int phmm_mixdom2_class_counts(const phmm_mixdom2_params *prm, int32_t
     if (!class_subs || !cnt_M || !cnt_I || !cnt_D || !class_match || !class_insert || !class_delete ||
         !classdist_counts)
         return pro_fail(PHMM_E_ARG, "phmm_mixdom2_class_counts: null device buffer");
-    const size_t smem = sizeof(double) * pk.K * pk.F * pk.C;
-    class_split_kernel<<<n_pairs, THREADS, smem, (cudaStream_t)stream>>>(
+    const SplitShape sh = split_shape(n_pairs, pk.K * pk.F, pk.C);
+    cudaError_t e = cudaSuccess;
+    if (sh.parts > 1)
+        e = cudaMemsetAsync(classdist_counts, 0, sizeof(double) * (size_t)n_pairs * pk.K * pk.F * pk.C, (cudaStream_t)stream);
+    if (e != cudaSuccess) return pro_fail(PHMM_E_CUDA, cudaGetErrorString(e));
+    class_split_kernel<<<dim3(n_pairs, sh.parts), sh.threads, sh.smem, (cudaStream_t)stream>>>(
         pk, class_subs, cnt_M, cnt_I, cnt_D, class_match, class_insert, class_delete, classdist_counts);
-    cudaError_t e = cudaGetLastError();
+    e = cudaGetLastError();
     if (e != cudaSuccess) return pro_fail(PHMM_E_CUDA, cudaGetErrorString(e));
     return PHMM_OK;
 }
@@ -1065,7 +1060,7 @@ extern "C" int phmm_mixdom2_chi_vjp(const phmm_mixdom2_params *prm, int32_t n_pa
 namespace pro {
 
 constexpr int HR_MAXA = 32;
-constexpr int HR_THREADS = 128;
+constexpr int HR_THREADS = 416;   // a thread per entry at 20 residues: the products' chains overlap across 13 warps
 
 struct HRClass {
     int A;
@@ -1147,11 +1142,12 @@ __global__ void __launch_bounds__(HR_THREADS) hr_kernel(const __grid_constant__ 
 
 // the same with the class blocks in device memory (hcs[c]; a captured graph
 // refreshes them by a copy before each replay)
-__global__ void __launch_bounds__(HR_THREADS) hr_kernel_dp(const HRClass *__restrict__ hcs, int c, int C,
+// blockIdx.y: the class
+__global__ void __launch_bounds__(HR_THREADS) hr_kernel_dp(const HRClass *__restrict__ hcs, int C,
                                                            const double *__restrict__ t,
                                                            const double *__restrict__ mc, double *__restrict__ W,
                                                            double *__restrict__ U) {
-    hr_kernel_body(hcs[c], c, C, t, mc, W, U);
+    hr_kernel_body(hcs[blockIdx.y], blockIdx.y, C, t, mc, W, U);
 }
 
 // Eigenvalues and orthonormal eigenvectors of a symmetric n x n matrix by the
@@ -1380,11 +1376,15 @@ extern "C" int phmm_mixdom2_class_counts_dp(const void *param_block, int32_t n_d
     if (!param_block || !class_subs || !cnt_M || !cnt_I || !cnt_D || !class_match || !class_insert ||
         !class_delete || !classdist_counts)
         return pro_fail(PHMM_E_ARG, "phmm_mixdom2_class_counts_dp: null device buffer");
-    const size_t smem = sizeof(double) * K * F * C;
-    class_split_kernel_dp<<<n_pairs, THREADS, smem, (cudaStream_t)stream>>>(
+    const SplitShape sh = split_shape(n_pairs, K * F, C);
+    cudaError_t e = cudaSuccess;
+    if (sh.parts > 1)
+        e = cudaMemsetAsync(classdist_counts, 0, sizeof(double) * (size_t)n_pairs * K * F * C, (cudaStream_t)stream);
+    if (e != cudaSuccess) return pro_fail(PHMM_E_CUDA, cudaGetErrorString(e));
+    class_split_kernel_dp<<<dim3(n_pairs, sh.parts), sh.threads, sh.smem, (cudaStream_t)stream>>>(
         reinterpret_cast<const Packed *>(param_block), class_subs, cnt_M, cnt_I, cnt_D, class_match, class_insert,
         class_delete, classdist_counts);
-    cudaError_t e = cudaGetLastError();
+    e = cudaGetLastError();
     if (e != cudaSuccess) return pro_fail(PHMM_E_CUDA, cudaGetErrorString(e));
     return PHMM_OK;
 }
@@ -1417,9 +1417,8 @@ extern "C" int phmm_holmes_rubin_dp(const void *block, int32_t n_classes, int32_
     if (n_pairs == 0) return PHMM_OK;
     if (!block || !t || !class_match_counts || !W || !U)
         return pro_fail(PHMM_E_ARG, "phmm_holmes_rubin_dp: null device buffer");
-    for (int c = 0; c < n_classes; ++c)
-        hr_kernel_dp<<<n_pairs, HR_THREADS, 0, (cudaStream_t)stream>>>(reinterpret_cast<const HRClass *>(block), c,
-                                                                       n_classes, t, class_match_counts, W, U);
+    hr_kernel_dp<<<dim3(n_pairs, n_classes), HR_THREADS, 0, (cudaStream_t)stream>>>(
+        reinterpret_cast<const HRClass *>(block), n_classes, t, class_match_counts, W, U);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return pro_fail(PHMM_E_CUDA, cudaGetErrorString(e));
     return PHMM_OK;
