@@ -45,7 +45,7 @@
 namespace {
 
 constexpr int TH = 32;             // rows per stripe == lanes per warp
-constexpr int HC = 32;             // halo chunk width (columns)
+constexpr int HC = 8;              // halo chunk width (columns): a stripe runs TH + HC columns behind the one above
 constexpr int MAXS = 168;          // max padded state slots (42 quads): the wide kernels
 constexpr int GMAXS = 64;          // max padded slots of the generic, warp and block kernels
 constexpr int MAXQ = MAXS / 4;
@@ -126,7 +126,7 @@ struct KParams {
 
 struct SmemLayout {
     int chi, chiE, tM, tI, tD, ring, raw, mx, halo, fst, ft, ut;  // float offsets
-    int ringE, haloE, fstE;                                         // int offsets
+    int ringE, haloE, fstE, used;                                   // int offsets
     int bins;                                                       // double offset
     int ys;                                                         // byte offset
     int bytes;
@@ -156,6 +156,7 @@ __host__ __device__ inline SmemLayout make_layout(int NS, int NQ, int G, int max
     L.ringE = o; o += 3 * TH;
     L.haloE = o; o += al4(2 * (HC + 1));
     if (bwd) { L.fstE = o; o += 2 * TH; } else { L.fstE = -1; }
+    L.used = o; o += al4(NS + 1);
     o = (o + 3) & ~3;
     if (bwd) { L.bins = o / 2; o += 2 * G * NBIN; } else { L.bins = -1; }
     int bytes = o * 4;
@@ -170,6 +171,22 @@ __device__ __forceinline__ float pow2f(int e) {
     if (e >= -126) return __int_as_float((min(e, 127) + 127) << 23);
     if (e >= -149) return __int_as_float(1 << (e + 149));
     return 0.0f;
+}
+
+// e with m 2^-e in [0.5, 1), for m > 0, and v 2^-e (exact, but for results below the normal range)
+__device__ __forceinline__ int exponent_of(float m) {
+    const int b = __float_as_int(m) >> 23;
+    if (b > 0 && b < 255) return b - 126;
+    int e;
+    frexpf(m, &e);
+    return e;
+}
+__device__ __forceinline__ float4 scale_down(float4 v, int e) {
+    if (e >= -126 && e <= 126) {
+        const float s = __int_as_float((127 - e) << 23);
+        return make_float4(v.x * s, v.y * s, v.z * s, v.w * s);
+    }
+    return make_float4(ldexpf(v.x, -e), ldexpf(v.y, -e), ldexpf(v.z, -e), ldexpf(v.w, -e));
 }
 
 __device__ __forceinline__ int ld_acquire(const int *p) {
@@ -282,6 +299,12 @@ __device__ void load_pair_model(const KParams &P, int p, const PairMeta &m, cons
         sm[L.tI + idx] = __ldg(eI + idx);
         sm[L.tD + idx] = __ldg(eD + idx);
     }
+    if (tid == 0) {   // the slots that hold a state, in order, and their number: the others add nothing to a sum
+        int *used = reinterpret_cast<int *>(sm) + L.used, n = 0;
+        for (int s = 0; s < NS; ++s)
+            if (P.slot_orig[s] >= 0) used[1 + n++] = s;
+        used[0] = n;
+    }
     unsigned char *ys = smb + L.ys;
     for (int j = tid; j <= m.Ly; j += nt) {
         int c = 0;
@@ -324,6 +347,62 @@ __device__ __forceinline__ float4 emit4(const float *sm, const EmitBase &eb, int
                        sm[eb.off[2] + add] * eb.mask[2], sm[eb.off[3] + add] * eb.mask[3]);
 }
 
+// The optional float64 tables are written by the wavefronts as pairs (float32
+// value, exponent) in place and turned into logarithms and posteriors by
+// tables_kernel afterwards, over all SMs: float64 logarithms and conversions
+// run on two lanes per SM, and inside a step they were half of it (one pair of
+// 150 x 160 at 5 states: forward 0.96 -> 0.46 ms, backward 2.05 -> 0.91 ms, the
+// table kernel 11 us; with 8-column halo chunks instead of 32, the sums over
+// occupied slots only and powers of two by bits 0.35 and 0.76 ms).  EMPTY (all ones) marks an entry no cell wrote.
+__device__ __forceinline__ void table_put(double *to, float v, int e) {
+    *reinterpret_cast<int2 *>(to) = make_int2(__float_as_int(v), e);
+}
+__device__ __forceinline__ bool table_empty(int2 w) { return w.x == -1 && w.y == -1; }
+
+// One pair per blockIdx.x, its table entries over blockIdx.y: log tables, and
+// posteriors with their sums by emitting state and residues.
+__global__ void __launch_bounds__(256) tables_kernel(const KParams P) {
+    extern __shared__ int16_t by_state[];       // [N] type, [N] group
+    const PairMeta m = P.meta[blockIdx.x];
+    const int N = P.N, p = blockIdx.x, G = P.G;
+    int16_t *type = by_state, *group = by_state + N;
+    for (int s = threadIdx.x; s < N; s += blockDim.x) type[s] = T_NONE;
+    __syncthreads();
+    for (int s = threadIdx.x; s < P.NS; s += blockDim.x)
+        if (P.slot_orig[s] >= 0) {
+            type[P.slot_orig[s]] = P.slot_type[s];
+            group[P.slot_orig[s]] = P.slot_group[s];
+        }
+    __syncthreads();
+    const int64_t n = (int64_t)(m.Lx + 1) * (m.Ly + 1) * N, base = m.tab_base * N;
+    for (int64_t idx = blockIdx.y * (int64_t)blockDim.x + threadIdx.x; idx < n; idx += (int64_t)gridDim.y * blockDim.x) {
+        for (int w = 0; w < 2; ++w) {
+            double *t = w == 0 ? P.F_log : P.B_log;
+            if (!t) continue;
+            const int2 v = reinterpret_cast<const int2 *>(t)[base + idx];
+            const float x = __int_as_float(v.x);
+            t[base + idx] = (!table_empty(v) && x > 0.f && v.y > EXP_NONE) ? log((double)x) + (double)v.y * LN2 : NEG_INF_LL;
+        }
+        if (P.post) {
+            const int2 v = reinterpret_cast<const int2 *>(P.post)[base + idx];
+            const float x = table_empty(v) ? 0.f : __int_as_float(v.x);
+            const double pv = (double)x;
+            P.post[base + idx] = P.beam_scale > 0.f ? fmin(pv, 1.0) : pv;
+            const int s = (int)(idx % N);
+            if (x != 0.f && type[s] >= T_M && type[s] <= T_D) {
+                const int64_t cell = idx / N;
+                const int i = (int)(cell / (m.Ly + 1)), j = (int)(cell % (m.Ly + 1));
+                const int a = i > 0 ? min((int)P.res[m.x_off + i - 1], 20) : 0;
+                const int b = j > 0 ? min((int)P.res[m.y_off + j - 1], 20) : 0;
+                const int64_t g = (int64_t)p * G + group[s];
+                if (type[s] == T_M) atomicAdd(P.cntM + g * 441 + a * 21 + b, pv);
+                else if (type[s] == T_I) atomicAdd(P.cntI + g * 21 + b, pv);
+                else atomicAdd(P.cntD + g * 21 + a, pv);
+            }
+        }
+    }
+}
+
 // ---------------------------------------------------------------- forward
 __device__ void forward_stripe(const KParams &P, int p, int si, const SmemLayout &L, float *sm,
                                unsigned char *smb, int *s_flag) {
@@ -359,6 +438,8 @@ __device__ void forward_stripe(const KParams &P, int p, int si, const SmemLayout
     int *haloE = reinterpret_cast<int *>(sm) + L.haloE;
     float *raw = sm + L.raw;
     float *mx = sm + L.mx;
+    const int *used = reinterpret_cast<int *>(sm) + L.used;
+    const int n_used = used[0];
     const int T_last = (nrows - 1) + Ly;
     const int qt = eb.type;
     bool aborted = false;
@@ -427,19 +508,12 @@ __device__ void forward_stripe(const KParams &P, int p, int si, const SmemLayout
             if (qt == T_D && hasD) { pp = pD; pst = stD; Ep = ED_; have = true; }
             float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
             if (have && Ep > EXP_NONE) {
-                for (int s = 0; s < NS; s += 4) {
-                    const float v0 = pp[(s + 0) * pst], v1 = pp[(s + 1) * pst];
-                    const float v2 = pp[(s + 2) * pst], v3 = pp[(s + 3) * pst];
-                    const float4 c0 = chi4[(s + 0) * NQ], c1 = chi4[(s + 1) * NQ];
-                    const float4 c2 = chi4[(s + 2) * NQ], c3 = chi4[(s + 3) * NQ];
+                for (int z = 1; z <= n_used; ++z) {
+                    const int s = used[z];
+                    const float v0 = pp[s * pst];
+                    const float4 c0 = chi4[s * NQ];
                     acc.x = fmaf(v0, c0.x, acc.x); acc.y = fmaf(v0, c0.y, acc.y);
                     acc.z = fmaf(v0, c0.z, acc.z); acc.w = fmaf(v0, c0.w, acc.w);
-                    acc.x = fmaf(v1, c1.x, acc.x); acc.y = fmaf(v1, c1.y, acc.y);
-                    acc.z = fmaf(v1, c1.z, acc.z); acc.w = fmaf(v1, c1.w, acc.w);
-                    acc.x = fmaf(v2, c2.x, acc.x); acc.y = fmaf(v2, c2.y, acc.y);
-                    acc.z = fmaf(v2, c2.z, acc.z); acc.w = fmaf(v2, c2.w, acc.w);
-                    acc.x = fmaf(v3, c3.x, acc.x); acc.y = fmaf(v3, c3.y, acc.y);
-                    acc.z = fmaf(v3, c3.z, acc.z); acc.w = fmaf(v3, c3.w, acc.w);
                 }
                 const float4 e = emit4(sm, eb, ys[j]);
                 const float sc = pow2f(Ep - Eref);
@@ -463,9 +537,8 @@ __device__ void forward_stripe(const KParams &P, int p, int si, const SmemLayout
             }
             int Ecell = EXP_NONE;
             if (mval > 0.0f) {
-                int e;
-                frexpf(mval, &e);
-                v = make_float4(ldexpf(v.x, -e), ldexpf(v.y, -e), ldexpf(v.z, -e), ldexpf(v.w, -e));
+                const int e = exponent_of(mval);
+                v = scale_down(v, e);
                 Ecell = Eref + e;
             } else {
                 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -496,9 +569,7 @@ __device__ void forward_stripe(const KParams &P, int p, int si, const SmemLayout
                 for (int u = 0; u < 4; ++u) {
                     const int os = P.slot_orig[4 * q + u];
                     if (os < 0) continue;
-                    const float x = f4get(v, u);
-                    P.F_log[cell * N + os] = (x > 0.f && Ecell > EXP_NONE)
-                        ? log((double)x) + (double)Ecell * LN2 : NEG_INF_LL;
+                    table_put(P.F_log + cell * N + os, f4get(v, u), Ecell);
                 }
             }
         }
@@ -608,6 +679,14 @@ __device__ void backward_stripe(const KParams &P, int p, int si, const SmemLayou
     float4 *ft4 = reinterpret_cast<float4 *>(sm + L.ft);
     float4 *ut4 = reinterpret_cast<float4 *>(sm + L.ut);
     const float4 *chiB4 = reinterpret_cast<const float4 *>(sm + L.chi) + q;  // chiB[k][4q..]
+    const int *used = reinterpret_cast<int *>(sm) + L.used;
+    int ubeg[4] = {1, 1, 1, 1};   // the M, I, D destinations' places in the list of used slots
+    for (int z = 1; z <= used[0]; ++z) {
+        const int k = used[z];
+        for (int ty = 0; ty < 3; ++ty)
+            if (k < P.kend[ty]) ubeg[ty + 1] = z + 1;
+    }
+    for (int ty = 1; ty < 4; ++ty) ubeg[ty] = max(ubeg[ty], ubeg[ty - 1]);
 
     // count-phase role: (source quad sq, dest quad kq, row group rg)
     const int npairs = NQ * NQ;
@@ -707,7 +786,8 @@ __device__ void backward_stripe(const KParams &P, int p, int si, const SmemLayou
                     const float *w = wp[ty];
                     const int st = ws[ty];
                     float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-                    for (int k = P.kbeg[ty]; k < P.kend[ty]; ++k) {
+                    for (int z = ubeg[ty]; z < ubeg[ty + 1]; ++z) {
+                        const int k = used[z];
                         const float wv = w[k * st];
                         const float4 c = chiB4[k * NQ];
                         a.x = fmaf(wv, c.x, a.x); a.y = fmaf(wv, c.y, a.y);
@@ -733,9 +813,8 @@ __device__ void backward_stripe(const KParams &P, int p, int si, const SmemLayou
             float4 b = make_float4(rw[0], rw[TH], rw[2 * TH], rw[3 * TH]);
             int Eb = EXP_NONE;
             if (mval > 0.0f) {
-                int e;
-                frexpf(mval, &e);
-                b = make_float4(ldexpf(b.x, -e), ldexpf(b.y, -e), ldexpf(b.z, -e), ldexpf(b.w, -e));
+                const int e = exponent_of(mval);
+                b = scale_down(b, e);
                 Eb = Eref + e;
             } else {
                 b = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -784,7 +863,7 @@ __device__ void backward_stripe(const KParams &P, int p, int si, const SmemLayou
             }
             // posteriors -> per-group character bins
             const float4 post4 = make_float4(ftv.x * b.x, ftv.y * b.y, ftv.z * b.z, ftv.w * b.w);
-            if (qt != T_NONE) {
+            if (qt != T_NONE && !P.post) {   // (the table kernel sums them from a posterior table)
                 for (int u = 0; u < 4; ++u) {
                     const int k = 4 * q + u;
                     const int kt = P.slot_type[k];
@@ -810,15 +889,8 @@ __device__ void backward_stripe(const KParams &P, int p, int si, const SmemLayou
                 for (int u = 0; u < 4; ++u) {
                     const int os = P.slot_orig[4 * q + u];
                     if (os < 0) continue;
-                    if (P.post) {
-                        const double pv = (double)f4get(post4, u);
-                        P.post[cell * N + os] = P.beam_scale > 0.f ? fmin(pv, 1.0) : pv;
-                    }
-                    if (P.B_log) {
-                        const float x = f4get(b, u);
-                        P.B_log[cell * N + os] = (x > 0.f && Eb > EXP_NONE)
-                            ? log((double)x) + (double)Eb * LN2 : NEG_INF_LL;
-                    }
+                    if (P.post) table_put(P.post + cell * N + os, f4get(post4, u), 0);
+                    if (P.B_log) table_put(P.B_log + cell * N + os, f4get(b, u), Eb);
                 }
             }
         }
@@ -909,12 +981,6 @@ __global__ void __launch_bounds__(512) backward_kernel(const KParams P) {
         const int2 w = P.items[it];
         backward_stripe(P, w.x, w.y, L, sm, smem_raw, &s_flag);
     }
-}
-
-__global__ void fill_f64(double *p, int64_t n, double v) {
-    for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < n;
-         idx += (int64_t)gridDim.x * blockDim.x)
-        p[idx] = v;
 }
 
 // Live column range of each stripe under a cell mask: one CTA per forward
@@ -1955,9 +2021,8 @@ int run_core(phmm_plan *plan, const phmm_batch *b, bool estep, double *ll, doubl
         CUDA_TRY(cudaMemsetAsync(cntI, 0, sizeof(double) * (size_t)P_ * G * 21, stream));
         CUDA_TRY(cudaMemsetAsync(cntD, 0, sizeof(double) * (size_t)P_ * G * 21, stream));
     }
-    if (F_log) { fill_f64<<<256, 256, 0, stream>>>(F_log, tab_cells * N, NEG_INF_LL); plan->launches++; }
-    if (B_log) { fill_f64<<<256, 256, 0, stream>>>(B_log, tab_cells * N, NEG_INF_LL); plan->launches++; }
-    if (post) CUDA_TRY(cudaMemsetAsync(post, 0, sizeof(double) * (size_t)tab_cells * N, stream));
+    for (double *t : {F_log, B_log, post})   // no cell has written an entry yet
+        if (t) CUDA_TRY(cudaMemsetAsync(t, 0xff, sizeof(double) * (size_t)tab_cells * N, stream));
 
     K.res = b->residues;
     K.meta = (const PairMeta *)d_meta;
@@ -2029,6 +2094,15 @@ int run_core(phmm_plan *plan, const phmm_batch *b, bool estep, double *ll, doubl
             CUDA_TRY(cudaGetLastError());
         }
         if (plan->timing) CUDA_TRY(cudaEventRecord(plan->ev[bwd ? 3 : 1], stream));
+        plan->launches++;
+    }
+    if (tables) {
+        int64_t most = 1;
+        for (int p = 0; p < b->n_pairs; ++p)
+            most = std::max(most, (int64_t)(b->Lx_host[p] + 1) * (b->Ly_host[p] + 1) * N);
+        tables_kernel<<<dim3(b->n_pairs, (unsigned)std::min<int64_t>(1024, (most + 255) / 256)), 256,
+                        2 * sizeof(int16_t) * N, stream>>>(K);
+        CUDA_TRY(cudaGetLastError());
         plan->launches++;
     }
     plan->timed_bwd = estep;

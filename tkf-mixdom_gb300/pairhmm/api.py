@@ -156,24 +156,23 @@ def _groups_from_table(log_emit, state_types, x, y):
     return groups, EM, EI, ED, mask
 
 
-def _run_single_tables(chi, st, groups, EM, EI, ED, x, y, forward_only=False, cell_mask=None, beam=0.0):
+def _run_single_tables(chi, st, groups, EM, EI, ED, x, y, tables='FBP', cell_mask=None, beam=0.0):
+    """One pair's E-step with the lattice tables named in `tables`: F, B (log forward and backward), P (posteriors)."""
     dev = _device()
     plan = get_plan(st, groups, EM.shape[0])
     b = _lib.make_batch([x], [y], np.asarray(chi)[None], np.asarray(EM)[None],
                         np.asarray(EI)[None], np.asarray(ED)[None], device=dev,
                         cell_masks=None if cell_mask is None else [cell_mask], beam_log_width=beam)
-    out = _lib.estep_tables(plan, b, want_F=True, want_B=not forward_only,
-                            want_post=not forward_only)
+    out = _lib.estep_tables(plan, b, want_F='F' in tables, want_B='B' in tables, want_post='P' in tables)
     Lx, Ly = len(x), len(y)
     N = len(st)
     res = {'ll': float(out['ll'][0]), 'status': int(out['status'][0]),
            'n_trans': out['n_trans'][0].cpu().numpy(),
            'cnt_M': out['cnt_M'][0].cpu().numpy(), 'cnt_I': out['cnt_I'][0].cpu().numpy(),
-           'cnt_D': out['cnt_D'][0].cpu().numpy(),
-           'F': out['log_F'].cpu().numpy().reshape(Lx + 1, Ly + 1, N)}
-    if not forward_only:
-        res['B'] = out['log_B'].cpu().numpy().reshape(Lx + 1, Ly + 1, N)
-        res['post'] = out['post'].cpu().numpy().reshape(Lx + 1, Ly + 1, N)
+           'cnt_D': out['cnt_D'][0].cpu().numpy()}
+    for key, name, want in (('F', 'log_F', 'F'), ('B', 'log_B', 'B'), ('post', 'post', 'P')):
+        if want in tables:
+            res[key] = out[name].cpu().numpy().reshape(Lx + 1, Ly + 1, N)
     return res
 
 
@@ -188,7 +187,7 @@ def forward_2d(log_trans, state_types, x_seq, y_seq, sub_matrix, pi):
     st = np.asarray(state_types)
     EM, EI, ED = _tkf_tables(sub_matrix, pi)
     r = _run_single_tables(_chi_from_log(log_trans), st, np.zeros(st.size, np.int32), EM, EI, ED,
-                           np.asarray(x_seq), np.asarray(y_seq), forward_only=True)
+                           np.asarray(x_seq), np.asarray(y_seq), tables='F')
     return r['ll'], r['F']
 
 
@@ -198,7 +197,7 @@ def backward_2d(log_trans, state_types, x_seq, y_seq, sub_matrix, pi):
     st = np.asarray(state_types)
     EM, EI, ED = _tkf_tables(sub_matrix, pi)
     r = _run_single_tables(_chi_from_log(log_trans), st, np.zeros(st.size, np.int32), EM, EI, ED,
-                           np.asarray(x_seq), np.asarray(y_seq))
+                           np.asarray(x_seq), np.asarray(y_seq), tables='B')
     return r['B']
 
 
@@ -223,7 +222,7 @@ def forward_backward_2d(log_trans, state_types, x_seq, y_seq, sub_matrix, pi,
         groups = np.zeros(st.size, np.int32)
         EM, EI, ED = _tkf_tables(sub_matrix, pi)
     r = _run_single_tables(_chi_from_log(log_trans), st, groups, EM, EI, ED, xr, yr,
-                           forward_only=forward_only, cell_mask=mask)
+                           tables='F' if forward_only else 'P', cell_mask=mask)
     if forward_only:
         return r['ll']
     post = np.zeros((pad_to_bin(Lx_arr) + 1, pad_to_bin(Ly_arr) + 1, st.size))
@@ -380,7 +379,7 @@ def forward_backward_2d_banded(log_trans, state_types, x_seq, y_seq, sub_matrix,
     groups = np.zeros(st.size, np.int32)
     plan = get_plan(st, groups, EM.shape[0])
     if not has_two_warp(plan):
-        r = _run_single_tables(chi, st, groups, EM, EI, ED, x, y, cell_mask=mask)
+        r = _run_single_tables(chi, st, groups, EM, EI, ED, x, y, tables='P', cell_mask=mask)
         return r['ll'], _to_band_layout(r['post'], band_center, W), r['n_trans']
     b = _lib.make_batch([x], [y], np.asarray(chi)[None], np.asarray(EM)[None], np.asarray(EI)[None],
                         np.asarray(ED)[None], device=_device(), cell_masks=[mask])
@@ -455,7 +454,7 @@ def _beam_run(log_trans, state_types, x_seq, y_seq, sub_matrix, pi, beam_log_wid
     # the beam module's emissions: log max(pi, 1e-30), log max(P, 1e-30)
     EM, EI, ED = pm.tables_per_domain(pm._t(np.asarray(sub_matrix, float))[None], pm._t(np.asarray(pi, float))[None])
     r = _run_single_tables(_chi_from_log(log_trans), st, np.zeros(st.size, np.int32), EM.numpy(), EI.numpy(),
-                           ED.numpy(), x, y, forward_only=forward_only, cell_mask=mask, beam=beam)
+                           ED.numpy(), x, y, tables='F' if forward_only else 'FP', cell_mask=mask, beam=beam)
     n_cells = int(np.count_nonzero(envelope)) - 1 if envelope is not None else (x.size + 1) * (y.size + 1) - 1
     return r, n_cells
 
@@ -669,7 +668,7 @@ def e_step(model, params, x, y):
         chi, st, groups, EM, EI, ED = _tkf_model(model, params)
     x = np.asarray(x)
     y = np.asarray(y)
-    r = _run_single_tables(chi, st, groups, EM, EI, ED, x, y)
+    r = _run_single_tables(chi, st, groups, EM, EI, ED, x, y, tables='P')
     post = r['post']
     Lx, Ly = len(x), len(y)
     mpost = post[1:, 1:, st == M].sum(axis=2)
