@@ -341,6 +341,22 @@ int phmm_mixdom2_chi_vjp_dirs(const phmm_mixdom2_params *prm);
 int phmm_mixdom2_chi_vjp(const phmm_mixdom2_params *prm, int32_t n_pairs, const double *t,
                          const double *grad_chi, double *grad, void *stream);
 
+/* The class substitution matrices and the emission tables of
+ * phmm_mixdom2_tables in float64 for the gradient path: class_subs [P][C][20][20],
+ * emit_M [P][KF][21][21], emit_I [P][KF][21] (emit_D is the same), and the
+ * vector-Jacobian product from their gradients (grad_I that of emit_I and emit_D
+ * together) to those of the times [P], class_S_exch [C][20][20] (its diagonal, which
+ * the tables do not read, gets 0), class_pis [C][20] and classdist [K][F][C]: the
+ * emission part of the gradient of mixdom2_log_prob and
+ * mixdom2_constrained_log_prob (train/vjp.py:463-510, 627-680, 1193-1437).  work:
+ * phmm_mixdom2_emissions_vjp_work doubles of device memory. */
+int phmm_mixdom2_emissions(const phmm_mixdom2_params *prm, int32_t n_pairs, const double *t, double *class_subs,
+                           double *emit_M, double *emit_I, void *stream);
+size_t phmm_mixdom2_emissions_vjp_work(const phmm_mixdom2_params *prm, int32_t n_pairs);
+int phmm_mixdom2_emissions_vjp(const phmm_mixdom2_params *prm, int32_t n_pairs, const double *t,
+                               const double *class_subs, const double *grad_M, const double *grad_I, double *work,
+                               double *grad_t, double *grad_S, double *grad_pis, double *grad_classdist, void *stream);
+
 /* 1D alignment-conditioned forward-backward (dp/hmm.py:127-250, 471-607):
  * along a fixed alignment the pair HMM is an HMM over the alignment columns.
  * Per pair p: columns off_host[p] .. off_host[p] + L_host[p] - 1 of emit
@@ -374,6 +390,15 @@ int phmm_fb1d_emissions(const phmm_model_desc *model, int32_t n_pairs, const int
                         const uint8_t *desc, const float *emit_M, const float *emit_I,
                         const float *emit_D, int32_t emit_per_pair, void *workspace,
                         size_t workspace_bytes, float *emit, int32_t *status_out, void *stream);
+
+/* Expected emission counts of alignments from the column posteriors of phmm_fb1d
+ * (columns, characters and model as phmm_fb1d_emissions): cnt_M [P][G][21][21],
+ * cnt_I / cnt_D [P][G][21] device float64, the posterior mass of the states of a
+ * column's type by group and characters.  workspace: at least 16 * n_pairs bytes. */
+int phmm_fb1d_counts(const phmm_model_desc *model, int32_t n_pairs, const int32_t *L_host, const int64_t *off_host,
+                     const uint8_t *cols, const uint8_t *anc, const uint8_t *desc, const float *posteriors,
+                     void *workspace, size_t workspace_bytes, double *cnt_M, double *cnt_I, double *cnt_D,
+                     void *stream);
 
 /* Viterbi path of each pair (dp/hmm.py:1976-2040), float64 log space: the
  * batch's sequences (residues, offsets, lengths; chi_per_pair / emit_per_pair

@@ -349,6 +349,28 @@ emit1d_kernel(const __grid_constant__ EmitDesc ed, const Meta *__restrict__ meta
     }
 }
 
+// Expected emission counts of the alignments: the posterior of every state at a
+// column of its type, summed by the state's group and the column's characters.
+// A warp per column; blockIdx.y takes columns of its own.
+__global__ void __launch_bounds__(256)
+count1d_kernel(const __grid_constant__ EmitDesc ed, const Meta *__restrict__ meta, const uint8_t *__restrict__ cols,
+               const uint8_t *__restrict__ anc, const uint8_t *__restrict__ desc, const float *__restrict__ post, int G,
+               double *__restrict__ cM, double *__restrict__ cI, double *__restrict__ cD) {
+    const int p = blockIdx.x, lane = threadIdx.x & 31, N = ed.N;
+    const Meta m = meta[p];
+    for (int l = blockIdx.y * 8 + (threadIdx.x >> 5); l < m.L; l += gridDim.y * 8) {
+        const int c = cols[m.off + l], a = min((int)anc[m.off + l], 20), b = min((int)desc[m.off + l], 20);
+        for (int s = lane; s < N; s += 32) {
+            if (c != ed.type[s] || c < 1 || c > 3) continue;
+            const double v = (double)post[(m.off + l) * N + s];
+            const int64_t g = (int64_t)p * G + ed.group[s];
+            if (c == 1) atomicAdd(cM + g * 441 + a * 21 + b, v);
+            else if (c == 2) atomicAdd(cI + g * 21 + b, v);
+            else atomicAdd(cD + g * 21 + a, v);
+        }
+    }
+}
+
 }  // namespace fb1
 
 static int fb1_fail(int code, const char *msg) {
@@ -474,6 +496,51 @@ extern "C" int phmm_fb1d_emissions(const phmm_model_desc *model, int32_t n_pairs
     for (const Meta &m : meta) most = std::max(most, (int)m.L);
     emit1d_kernel<<<dim3(n_pairs, std::min(16, (most + 31) / 32)), 256, 0, st>>>(ed, (const Meta *)workspace, cols, anc, desc, emit_M, emit_I, emit_D,
                                           emit_per_pair, G, emit, status_out);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return fb1_fail(PHMM_E_CUDA, cudaGetErrorString(e));
+    return PHMM_OK;
+}
+
+extern "C" int phmm_fb1d_counts(const phmm_model_desc *model, int32_t n_pairs, const int32_t *L_host,
+                                const int64_t *off_host, const uint8_t *cols, const uint8_t *anc, const uint8_t *desc,
+                                const float *posteriors, void *workspace, size_t workspace_bytes, double *cnt_M,
+                                double *cnt_I, double *cnt_D, void *stream) {
+    using namespace fb1;
+    if (!model || !model->state_types || !model->state_group)
+        return fb1_fail(PHMM_E_ARG, "phmm_fb1d_counts: bad model description");
+    const int N = model->n_states, G = model->n_groups;
+    if (N < 2 || N > MAXN) return fb1_fail(PHMM_E_ARG, "phmm_fb1d_counts: n_states must be in 2..64");
+    if (n_pairs < 0) return fb1_fail(PHMM_E_ARG, "phmm_fb1d_counts: negative n_pairs");
+    if (n_pairs == 0) return PHMM_OK;
+    if (!L_host || !off_host || !cols || !anc || !desc || !posteriors || !workspace || !cnt_M || !cnt_I || !cnt_D)
+        return fb1_fail(PHMM_E_ARG, "phmm_fb1d_counts: null pointer");
+    if (workspace_bytes < sizeof(Meta) * (size_t)n_pairs)
+        return fb1_fail(PHMM_E_ARG, "phmm_fb1d_counts: workspace too small");
+    EmitDesc ed;
+    std::memset(&ed, 0, sizeof(ed));
+    ed.N = N;
+    for (int s = 0; s < N; ++s) {
+        ed.type[s] = model->state_types[s];
+        ed.group[s] = (int8_t)model->state_group[s];
+        if (model->state_group[s] < 0 || model->state_group[s] >= G)
+            return fb1_fail(PHMM_E_ARG, "phmm_fb1d_counts: state group out of range");
+    }
+    std::vector<Meta> meta(n_pairs);
+    int most = 1;
+    for (int p = 0; p < n_pairs; ++p) {
+        if (L_host[p] < 0 || off_host[p] < 0) return fb1_fail(PHMM_E_ARG, "phmm_fb1d_counts: negative length");
+        meta[p] = Meta{off_host[p], L_host[p], 0};
+        most = std::max(most, (int)L_host[p]);
+    }
+    cudaStream_t st = (cudaStream_t)stream;
+    const size_t PG = (size_t)n_pairs * G;
+    cudaError_t e = cudaMemcpyAsync(workspace, meta.data(), sizeof(Meta) * n_pairs, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(cnt_M, 0, sizeof(double) * PG * 441, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(cnt_I, 0, sizeof(double) * PG * 21, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(cnt_D, 0, sizeof(double) * PG * 21, st);
+    if (e != cudaSuccess) return fb1_fail(PHMM_E_CUDA, cudaGetErrorString(e));
+    count1d_kernel<<<dim3(n_pairs, std::min(16, (most + 31) / 32)), 256, 0, st>>>(
+        ed, (const Meta *)workspace, cols, anc, desc, posteriors, G, cnt_M, cnt_I, cnt_D);
     e = cudaGetLastError();
     if (e != cudaSuccess) return fb1_fail(PHMM_E_CUDA, cudaGetErrorString(e));
     return PHMM_OK;

@@ -547,13 +547,14 @@ expm_kernel_dp(const Packed *__restrict__ prm, const double *__restrict__ ts, do
 }
 
 // ---------------------------------------------------------------- emission tables
-__device__ __forceinline__ void tables_kernel_body(const Packed &prm, const double *__restrict__ csubs, float *__restrict__ EM,
-              float *__restrict__ EI, float *__restrict__ ED) {
+template <class R>
+__device__ __forceinline__ void tables_kernel_body(const Packed &prm, const double *__restrict__ csubs, R *__restrict__ EM,
+              R *__restrict__ EI, R *__restrict__ ED) {
     const int p = blockIdx.x, tid = threadIdx.x;
     const int C = prm.C, G = prm.K * prm.F;
     const double *cd = prm.v + prm.o_cd, *pis = prm.v + prm.o_pis;
     const double *Pp = csubs + (size_t)p * C * NA * NA;
-    float *em = EM + (size_t)p * G * 441;
+    R *em = EM + (size_t)p * G * 441;
     for (int idx = tid; idx < G * 441; idx += blockDim.x) {
         const int g = idx / 441, a = (idx / 21) % 21, bb = idx % 21;
         double s = 0.0;
@@ -562,14 +563,14 @@ __device__ __forceinline__ void tables_kernel_body(const Packed &prm, const doub
             const double ls = (a < NA && bb < NA) ? fmax(Pp[(c * NA + a) * NA + bb], 1e-30) : 1.0;
             s += cd[g * C + c] * (lp * ls);
         }
-        em[idx] = (float)s;
+        em[idx] = (R)s;
     }
     for (int idx = tid; idx < G * 21; idx += blockDim.x) {
         const int g = idx / 21, a = idx % 21;
         double s = 0.0;
         for (int c = 0; c < C; ++c) s += cd[g * C + c] * (a < NA ? fmax(pis[c * NA + a], 1e-30) : 1.0);
-        EI[(size_t)p * G * 21 + idx] = (float)s;
-        ED[(size_t)p * G * 21 + idx] = (float)s;
+        EI[(size_t)p * G * 21 + idx] = (R)s;
+        if (ED) ED[(size_t)p * G * 21 + idx] = (R)s;
     }
 }
 
@@ -583,6 +584,213 @@ tables_kernel(const __grid_constant__ Packed prm, const double *__restrict__ csu
 __global__ void __launch_bounds__(THREADS)
 tables_kernel_dp(const Packed *__restrict__ prm, const double *__restrict__ csubs, float *__restrict__ EM, float *__restrict__ EI, float *__restrict__ ED) {
     tables_kernel_body(*prm, csubs, EM, EI, ED);
+}
+
+// float64 tables for the gradient path (EI = ED)
+__global__ void __launch_bounds__(THREADS)
+tables64_kernel(const __grid_constant__ Packed prm, const double *__restrict__ csubs, double *__restrict__ EM, double *__restrict__ EI) {
+    tables_kernel_body<double>(prm, csubs, EM, EI, nullptr);
+}
+
+// ---------------------------------------------------------------- emission tables, adjoint
+// From the gradients of the float64 tables (gM [P][G][21][21], g1 [P][G][21] of
+// EI = ED) to those of t, the exchangeabilities, the frequencies and classdist.
+//
+// emissions_vjp_kernel: one CTA per (pair, class).  With W[a][b] = sum_g w[g][c]
+// gM[g][a][b], the table's share of P_c is lp[a] W[a][b]; its adjoint through
+// exp(X), X = t Q_c, is the Frechet derivative of exp at X^T in that direction,
+// carried through the same polynomial and squarings as the matrix itself (each
+// product A B by A dB + dA B).  Three times the products of expm_kernel bound it:
+// 128 matrices at times up to 2 take 98 us.  The tensor library's exponential and
+// its differentiation in a 40 x 40 block form took 1.4 ms of the device and 6 ms of
+// host time for the same (60 launches).
+// emissions_finish_kernel sums the pairs' shares.
+__device__ __forceinline__ void mm20d(double *C, const double *A1, const double *B1, const double *A2, const double *B2,
+                                      const double *c = nullptr, const double *X = nullptr, const double *X2 = nullptr,
+                                      const double *X3 = nullptr) {   // A1 B1 + A2 B2 (+ c1 X + c2 X2 + c3 X3)
+    for (int idx = threadIdx.x; idx < NA * NA; idx += blockDim.x) {
+        const int i = idx / NA, j = idx % NA;
+        double s = 0.0, u = 0.0;
+#pragma unroll
+        for (int k = 0; k < NA; ++k) {
+            s += A1[i * NA + k] * B1[k * NA + j];
+            u += A2[i * NA + k] * B2[k * NA + j];
+        }
+        s += u;
+        if (c) s += c[1] * X[idx] + c[2] * X2[idx] + c[3] * X3[idx];
+        C[idx] = s;
+    }
+    __syncthreads();
+}
+
+// gQ [P][C][20][20], gpi [P][C][20], gcd [P][G][C], gt [P][C]: the pair's and class's shares
+__global__ void __launch_bounds__(THREADS)
+emissions_vjp_kernel(const __grid_constant__ Packed prm, const double *__restrict__ ts, const double *__restrict__ csubs,
+                     const double *__restrict__ gM, const double *__restrict__ g1, double *__restrict__ gQ,
+                     double *__restrict__ gpi, double *__restrict__ gcd, double *__restrict__ gt) {
+    constexpr int n = NA, nn = NA * NA;
+    __shared__ double X[nn], X2[nn], X3[nn], X4[nn], W1[nn], W2[nn];
+    __shared__ double E[nn], E2[nn], E3[nn], E4[nn], V1[nn], V2[nn];
+    __shared__ double lp[21], colsum[n], red[THREADS / 32];
+    __shared__ int n_sq, n_deg;
+    const int C = prm.C, G = prm.K * prm.F, p = blockIdx.x / C, c = blockIdx.x % C, tid = threadIdx.x;
+    const double t = ts[p];
+    const double *Sx = prm.v + prm.o_S + (size_t)c * nn, *pi = prm.v + prm.o_pis + c * n, *cd = prm.v + prm.o_cd;
+    const double *Pp = csubs + ((size_t)p * C + c) * nn;
+    const double *gm = gM + (size_t)p * G * 441, *g1p = g1 + (size_t)p * G * 21;
+    if (tid < 21) lp[tid] = tid < n ? fmax(pi[tid], 1e-30) : 1.0;
+    // X^T (unscaled) into X: X[b][a] = t Q[a][b]
+    for (int idx = tid; idx < nn; idx += blockDim.x) {
+        const int a = idx / n, b = idx % n;
+        W1[idx] = a == b ? 0.0 : Sx[idx] * pi[b];
+    }
+    __syncthreads();
+    if (tid < n) {
+        double s = 0.0;
+        for (int b = 0; b < n; ++b) s += W1[tid * n + b];
+        W1[tid * n + tid] = -s;
+    }
+    __syncthreads();
+    if (tid < n) {
+        double s = 0.0;
+        for (int a = 0; a < n; ++a) s += fabs(W1[a * n + tid]);
+        colsum[tid] = s * fabs(t);
+    }
+    __syncthreads();
+    if (tid == 0) {
+        double nrm = 0.0;
+        for (int b = 0; b < n; ++b) nrm = fmax(nrm, colsum[b]);
+        int s = 0;
+        if (nrm > THETA16) s = (int)ceil(log2(nrm / THETA16));
+        n_sq = s < 0 ? 0 : (s > 60 ? 60 : s);
+        n_deg = nrm <= THETA8 ? 8 : nrm <= THETA12 ? 12 : 16;
+    }
+    __syncthreads();
+    const int s = n_sq, m = n_deg;
+    for (int idx = tid; idx < nn; idx += blockDim.x) X[idx] = ldexp(W1[(idx % n) * n + idx / n] * t, -s);
+    __syncthreads();
+    // the table's adjoint: direction E = lp[a] W[a][b] (where P is not at its floor), frequencies, class weights
+    for (int idx = tid; idx < 441; idx += blockDim.x) {
+        const int a = idx / 21, b = idx % 21;
+        double w = 0.0;
+        for (int g = 0; g < G; ++g) w += cd[g * C + c] * gm[(size_t)g * 441 + idx];
+        if (a < n && b < n) E[a * n + b] = Pp[a * n + b] >= 1e-30 ? ldexp(lp[a] * w, -s) : 0.0;
+        if (a < n && b == n) colsum[a] = w;     // the wildcard column, whose factor is 1
+    }
+    __syncthreads();
+    if (tid < n) {
+        double w = colsum[tid];
+        for (int b = 0; b < n; ++b) {
+            const double P_ = Pp[tid * n + b];
+            double v = 0.0;
+            for (int g = 0; g < G; ++g) v += cd[g * C + c] * gm[(size_t)g * 441 + tid * 21 + b];
+            w += v * fmax(P_, 1e-30);
+        }
+        for (int g = 0; g < G; ++g) w += cd[g * C + c] * g1p[g * 21 + tid];
+        gpi[((size_t)p * C + c) * n + tid] = pi[tid] >= 1e-30 ? w : 0.0;
+    }
+    for (int g = tid >> 5; g < G; g += THREADS / 32) {   // a warp per group
+        double v = 0.0;
+        for (int idx = tid & 31; idx < 441 + 21; idx += 32) {
+            if (idx < 441) {
+                const int a = idx / 21, b = idx % 21;
+                v += gm[(size_t)g * 441 + idx] * (lp[a] * (a < n && b < n ? fmax(Pp[a * n + b], 1e-30) : 1.0));
+            } else {
+                v += g1p[g * 21 + idx - 441] * lp[idx - 441];
+            }
+        }
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if ((tid & 31) == 0) gcd[((size_t)p * G + g) * C + c] = v;
+    }
+    // exp and its derivative
+    mm20(X2, X, X);
+    mm20d(E2, X, E, E, X);
+    mm20(X3, X2, X);
+    mm20d(E3, X2, E, E2, X);
+    mm20(X4, X2, X2);
+    mm20d(E4, X2, E2, E2, X2);
+    for (int idx = tid; idx < nn; idx += blockDim.x) {
+        const double *f = INV_FACT + m - 4;
+        W1[idx] = (idx / n == idx % n ? f[0] : 0.0) + f[1] * X[idx] + f[2] * X2[idx] + f[3] * X3[idx] + f[4] * X4[idx];
+        V1[idx] = f[1] * E[idx] + f[2] * E2[idx] + f[3] * E3[idx] + f[4] * E4[idx];
+    }
+    __syncthreads();
+    double *w = W1, *wn = W2, *v = V1, *vn = V2;
+    auto swap = [&]() {
+        double *a = w, *b = v;
+        w = wn; v = vn;
+        wn = a; vn = b;
+    };
+    for (int j = m / 4 - 2; j >= 0; --j) {
+        mm20d(vn, w, E4, v, X4, INV_FACT + 4 * j, E, E2, E3);
+        mm20(wn, w, X4, INV_FACT + 4 * j, X, X2, X3);
+        swap();
+    }
+    for (int k = 0; k < s; ++k) {
+        mm20d(vn, w, v, v, w);
+        mm20(wn, w, w);
+        swap();
+    }
+    // v[a][b] = dL / d(t Q)[a][b]
+    double dt = 0.0;
+    for (int idx = tid; idx < nn; idx += blockDim.x) {
+        const int a = idx / n, b = idx % n;
+        gQ[((size_t)p * C + c) * nn + idx] = t * v[idx];
+        dt += v[idx] * (a == b ? 0.0 : Sx[idx] * pi[b]);
+        // the diagonal of Q is minus its row: every entry also takes the diagonal's share
+        dt -= a == b ? 0.0 : v[a * n + a] * (Sx[idx] * pi[b]);
+    }
+    for (int o = 16; o > 0; o >>= 1) dt += __shfl_xor_sync(0xffffffffu, dt, o);
+    if ((tid & 31) == 0) red[tid >> 5] = dt;
+    __syncthreads();
+    if (tid == 0) {
+        double q = 0.0;
+        for (int i = 0; i < THREADS / 32; ++i) q += red[i];
+        gt[(size_t)p * C + c] = q;
+    }
+}
+
+// Sums over the pairs: blockIdx.x < C: a class's exchangeabilities and
+// frequencies; the last block: classdist and the times.
+__global__ void __launch_bounds__(512)
+emissions_finish_kernel(const __grid_constant__ Packed prm, int P, const double *__restrict__ gQ,
+                        const double *__restrict__ gpi, const double *__restrict__ gcd, const double *__restrict__ gt,
+                        double *__restrict__ out_t, double *__restrict__ out_S, double *__restrict__ out_pi,
+                        double *__restrict__ out_cd) {
+    constexpr int n = NA, nn = NA * NA;
+    __shared__ double q[nn];
+    const int C = prm.C, G = prm.K * prm.F, c = blockIdx.x, tid = threadIdx.x;
+    if (c == C) {
+        for (int i = tid; i < G * C; i += blockDim.x) {
+            double s = 0.0;
+            for (int p = 0; p < P; ++p) s += gcd[(size_t)p * G * C + i];
+            out_cd[i] = s;
+        }
+        for (int p = tid; p < P; p += blockDim.x) {
+            double s = 0.0;
+            for (int k = 0; k < C; ++k) s += gt[(size_t)p * C + k];
+            out_t[p] = s;
+        }
+        return;
+    }
+    const double *Sx = prm.v + prm.o_S + (size_t)c * nn, *pi = prm.v + prm.o_pis + c * n;
+    for (int i = tid; i < nn; i += blockDim.x) {
+        double s = 0.0;
+        for (int p = 0; p < P; ++p) s += gQ[((size_t)p * C + c) * nn + i];
+        q[i] = s;
+    }
+    __syncthreads();
+    for (int i = tid; i < nn; i += blockDim.x) {
+        const int a = i / n, b = i % n;
+        out_S[(size_t)c * nn + i] = a == b ? 0.0 : (q[i] - q[a * n + a]) * pi[b];
+    }
+    if (tid < n) {
+        double s = 0.0;
+        for (int a = 0; a < n; ++a)
+            if (a != tid) s += (q[a * n + tid] - q[a * n + a]) * Sx[a * n + tid];
+        for (int p = 0; p < P; ++p) s += gpi[((size_t)p * C + c) * n + tid];
+        out_pi[c * n + tid] = s;
+    }
 }
 
 // ---------------------------------------------------------------- class split (epilogue)
@@ -915,6 +1123,52 @@ static int mixdom2_tables(const phmm_mixdom2_params *prm, int32_t n_pairs, const
     chi_kernel<<<n_pairs, THREADS, chi_smem, st>>>(pk, t, N, chi, nullptr, nest);
     expm_kernel<<<n_pairs * C, THREADS, 0, st>>>(pk, t, class_subs);
     tables_kernel<<<n_pairs, THREADS, 0, st>>>(pk, class_subs, emit_M, emit_I, emit_D);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return pro_fail(PHMM_E_CUDA, cudaGetErrorString(e));
+    return PHMM_OK;
+}
+
+extern "C" int phmm_mixdom2_emissions(const phmm_mixdom2_params *prm, int32_t n_pairs, const double *t,
+                                      double *class_subs, double *emit_M, double *emit_I, void *stream) {
+    using namespace pro;
+    Packed pk;
+    int rc = pack_params(prm, pk, "phmm_mixdom2_emissions");
+    if (rc) return rc;
+    if (n_pairs < 0) return pro_fail(PHMM_E_ARG, "phmm_mixdom2_emissions: negative n_pairs");
+    if (n_pairs == 0) return PHMM_OK;
+    if (!t || !class_subs || !emit_M || !emit_I)
+        return pro_fail(PHMM_E_ARG, "phmm_mixdom2_emissions: null device buffer");
+    cudaStream_t st = (cudaStream_t)stream;
+    expm_kernel<<<n_pairs * pk.C, THREADS, 0, st>>>(pk, t, class_subs);
+    tables64_kernel<<<n_pairs, THREADS, 0, st>>>(pk, class_subs, emit_M, emit_I);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return pro_fail(PHMM_E_CUDA, cudaGetErrorString(e));
+    return PHMM_OK;
+}
+
+extern "C" size_t phmm_mixdom2_emissions_vjp_work(const phmm_mixdom2_params *prm, int32_t n_pairs) {
+    if (!prm || n_pairs < 0 || prm->n_classes < 0) return 0;
+    const size_t C = prm->n_classes, G = (size_t)prm->n_dom * prm->n_frag;
+    return (size_t)n_pairs * (C * (pro::NA * pro::NA + pro::NA + 1) + G * C);
+}
+
+extern "C" int phmm_mixdom2_emissions_vjp(const phmm_mixdom2_params *prm, int32_t n_pairs, const double *t,
+                                          const double *class_subs, const double *grad_M, const double *grad_I,
+                                          double *work, double *grad_t, double *grad_S, double *grad_pis,
+                                          double *grad_classdist, void *stream) {
+    using namespace pro;
+    Packed pk;
+    int rc = pack_params(prm, pk, "phmm_mixdom2_emissions_vjp");
+    if (rc) return rc;
+    if (n_pairs < 1) return pro_fail(PHMM_E_ARG, "phmm_mixdom2_emissions_vjp: need a pair");
+    if (!t || !class_subs || !grad_M || !grad_I || !work || !grad_t || !grad_S || !grad_pis || !grad_classdist)
+        return pro_fail(PHMM_E_ARG, "phmm_mixdom2_emissions_vjp: null device buffer");
+    const size_t PC = (size_t)n_pairs * pk.C;
+    double *gQ = work, *gpi = gQ + PC * NA * NA, *gt = gpi + PC * NA, *gcd = gt + PC;
+    cudaStream_t st = (cudaStream_t)stream;
+    emissions_vjp_kernel<<<n_pairs * pk.C, THREADS, 0, st>>>(pk, t, class_subs, grad_M, grad_I, gQ, gpi, gcd, gt);
+    emissions_finish_kernel<<<pk.C + 1, 512, 0, st>>>(pk, n_pairs, gQ, gpi, gcd, gt, grad_t, grad_S, grad_pis,
+                                                      grad_classdist);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return pro_fail(PHMM_E_CUDA, cudaGetErrorString(e));
     return PHMM_OK;

@@ -24,7 +24,8 @@ EXPORTS = ('phmm_plan_create', 'phmm_plan_destroy', 'phmm_forward', 'phmm_estep'
            'phmm_last_variant', 'phmm_last_launch_count',
            'phmm_last_error', 'phmm_version', 'phmm_mixdom2_class_subs_count', 'phmm_mixdom2_tables',
            'phmm_mixdom2_class_counts', 'phmm_tkf92_tables', 'phmm_tkf92_bdi', 'phmm_mixdom2_chi',
-           'phmm_mixdom2_chi_vjp_dirs', 'phmm_mixdom2_chi_vjp', 'phmm_fb1d_workspace_bytes', 'phmm_fb1d',
+           'phmm_mixdom2_chi_vjp_dirs', 'phmm_mixdom2_chi_vjp', 'phmm_mixdom2_emissions',
+           'phmm_mixdom2_emissions_vjp_work', 'phmm_mixdom2_emissions_vjp', 'phmm_fb1d_counts', 'phmm_fb1d_workspace_bytes', 'phmm_fb1d',
            'phmm_fb1d_emissions', 'phmm_viterbi_workspace_bytes', 'phmm_viterbi', 'phmm_holmes_rubin',
            'phmm_sample_workspace_bytes', 'phmm_sample_paths', 'phmm_pairs_count', 'phmm_pairs_decode',
            'phmm_estep_ws_prepare', 'phmm_estep_ws_launch', 'phmm_mixdom2_param_block_bytes',
@@ -159,6 +160,15 @@ def load(path=None):
     lib.phmm_mixdom2_chi_vjp.restype = ctypes.c_int
     lib.phmm_tkf92_tables.argtypes = [ctypes.POINTER(Tkf92Params), ctypes.c_int32] + [vp] * 7
     lib.phmm_tkf92_tables.restype = ctypes.c_int
+    lib.phmm_mixdom2_emissions.argtypes = [ctypes.POINTER(MixDom2Params), ctypes.c_int32] + [vp] * 5
+    lib.phmm_mixdom2_emissions.restype = ctypes.c_int
+    lib.phmm_mixdom2_emissions_vjp_work.argtypes = [ctypes.POINTER(MixDom2Params), ctypes.c_int32]
+    lib.phmm_mixdom2_emissions_vjp_work.restype = ctypes.c_size_t
+    lib.phmm_mixdom2_emissions_vjp.argtypes = [ctypes.POINTER(MixDom2Params), ctypes.c_int32] + [vp] * 10
+    lib.phmm_mixdom2_emissions_vjp.restype = ctypes.c_int
+    lib.phmm_fb1d_counts.argtypes = [ctypes.POINTER(ModelDesc), ctypes.c_int32, ctypes.POINTER(ctypes.c_int32),
+                                     ctypes.POINTER(ctypes.c_int64)] + [vp] * 5 + [ctypes.c_size_t] + [vp] * 4
+    lib.phmm_fb1d_counts.restype = ctypes.c_int
     lib.phmm_tkf92_bdi.argtypes = [ctypes.c_double] * 3 + [ctypes.c_int32] + [vp] * 5
     lib.phmm_tkf92_bdi.restype = ctypes.c_int
     lib.phmm_fb1d_workspace_bytes.argtypes = [ctypes.POINTER(Fb1dBatch), ctypes.POINTER(ctypes.c_size_t)]
@@ -772,6 +782,31 @@ class MixDom2Prologue:
                                              ctypes.c_void_p(s.cuda_stream)), 'phmm_mixdom2_chi_vjp')
         return out
 
+    def emissions(self, t, stream=None):
+        """phmm_mixdom2_emissions: (EM [P,G,21,21], EI [P,G,21], csubs [P,C,20,20]) float64 for device times t [P]."""
+        P, f64 = t.numel(), torch.float64
+        csubs = torch.empty(P, self.C, self.A, self.A, dtype=f64, device=t.device)
+        EM = torch.empty(P, self.G, 21, 21, dtype=f64, device=t.device)
+        EI = torch.empty(P, self.G, 21, dtype=f64, device=t.device)
+        s = stream if stream is not None else torch.cuda.current_stream(t.device)
+        _check(self.lib.phmm_mixdom2_emissions(ctypes.byref(self.struct), P, _ptr(t), _ptr(csubs), _ptr(EM), _ptr(EI),
+                                               ctypes.c_void_p(s.cuda_stream)), 'phmm_mixdom2_emissions')
+        return EM, EI, csubs
+
+    def emissions_vjp(self, t, csubs, grad_M, grad_I, stream=None):
+        """phmm_mixdom2_emissions_vjp: gradients of (t [P], class_S_exch, class_pis, classdist) from those of
+        emissions()'s tables."""
+        P, f64 = t.numel(), torch.float64
+        new = lambda *sh: torch.empty(*sh, dtype=f64, device=t.device)
+        gM, gI = grad_M.to(f64).contiguous(), grad_I.to(f64).contiguous()
+        out = (new(P), new(self.C, self.A, self.A), new(self.C, self.A), new(self.K, self.F, self.C))
+        work = new(self.lib.phmm_mixdom2_emissions_vjp_work(ctypes.byref(self.struct), P))
+        s = stream if stream is not None else torch.cuda.current_stream(t.device)
+        _check(self.lib.phmm_mixdom2_emissions_vjp(
+            ctypes.byref(self.struct), P, _ptr(t), _ptr(csubs), _ptr(gM), _ptr(gI), _ptr(work), *map(_ptr, out),
+            ctypes.c_void_p(s.cuda_stream)), 'phmm_mixdom2_emissions_vjp')
+        return out
+
     def __call__(self, ts, device='cuda', stream=None, with_nest=False):
         """(chi, EM, EI, ED, csubs) on the device for per-pair times ts; with
         with_nest, the factored record (phmm_batch.nest) appended, built by
@@ -974,6 +1009,28 @@ def fb1d_emissions(state_types, groups, G, L, off, cols, anc, desc, emit_M, emit
                                    ctypes.c_size_t(ws.numel()), _ptr(out), _ptr(status),
                                    ctypes.c_void_p(s.cuda_stream)), 'phmm_fb1d_emissions')
     return out, status
+
+
+def fb1d_counts(state_types, groups, G, L, off, cols, anc, desc, posteriors, stream=None):
+    """phmm_fb1d_counts: (cnt_M [P,G,21,21], cnt_I, cnt_D [P,G,21]) float64 from the column posteriors [cols, N]
+    (device float32) of alignments (device uint8 cols / anc / desc)."""
+    lib = load()
+    st_arr = np.ascontiguousarray(np.asarray(state_types, np.int8))
+    gr = np.ascontiguousarray(np.asarray(groups, np.int32))
+    desc_m = ModelDesc(st_arr.size, st_arr.ctypes.data_as(ctypes.POINTER(ctypes.c_int8)),
+                       gr.ctypes.data_as(ctypes.POINTER(ctypes.c_int32)), int(G))
+    L = np.ascontiguousarray(np.asarray(L, np.int32))
+    off = np.ascontiguousarray(np.asarray(off, np.int64))
+    P, dev, f64 = L.size, cols.device, torch.float64
+    out = (torch.empty(P, int(G), 21, 21, dtype=f64, device=dev), torch.empty(P, int(G), 21, dtype=f64, device=dev),
+           torch.empty(P, int(G), 21, dtype=f64, device=dev))
+    ws = torch.empty(max(16 * P, 256), dtype=torch.uint8, device=dev)
+    s = stream if stream is not None else torch.cuda.current_stream(dev)
+    _check(lib.phmm_fb1d_counts(ctypes.byref(desc_m), P, L.ctypes.data_as(ctypes.POINTER(ctypes.c_int32)),
+                                off.ctypes.data_as(ctypes.POINTER(ctypes.c_int64)), _ptr(cols), _ptr(anc), _ptr(desc),
+                                _ptr(posteriors), _ptr(ws), ctypes.c_size_t(ws.numel()), *map(_ptr, out),
+                                ctypes.c_void_p(s.cuda_stream)), 'phmm_fb1d_counts')
+    return out
 
 
 def viterbi(state_types, groups, G, xs, ys, log_chi, log_M, log_I, log_D, device='cuda', stream=None,

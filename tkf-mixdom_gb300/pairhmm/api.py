@@ -845,35 +845,14 @@ class ConstrainedLogLik(torch.autograd.Function):
                           if lens.sum() else np.zeros(1, np.int64))
         c_all, a_all, d_all = cat(cols), cat(ancs), cat(descs)
         to_u8 = lambda a: torch.from_numpy(np.clip(a, 0, 255).astype(np.uint8)).to(dev)
+        c_dev, a_dev, d_dev = to_u8(c_all), to_u8(a_all), to_u8(d_all)
         f32 = lambda v: v.detach().to(torch.float32).contiguous()
         per_pair = EM.shape[0] == P
-        emit, st1 = _lib.fb1d_emissions(st, gr, G, lens, off, to_u8(c_all), to_u8(a_all), to_u8(d_all),
-                                        f32(EM), f32(EI), f32(ED), per_pair)
+        emit, st1 = _lib.fb1d_emissions(st, gr, G, lens, off, c_dev, a_dev, d_dev, f32(EM), f32(EI), f32(ED), per_pair)
         ll, nt, post, st2 = _lib.fb1d(N, lens, off, emit, f32(chi), chi.shape[0] == P and chi.dim() == 3, 0, 1,
                                       posteriors=True)
         # character counts per pair from the column posteriors
-        ncol = int(lens.sum())
-        pair_of = torch.as_tensor(np.repeat(np.arange(P), lens), device=dev)
-        cM = torch.zeros(P * G * 441, dtype=torch.float64, device=dev)
-        cI = torch.zeros(P * G * 21, dtype=torch.float64, device=dev)
-        cD = torch.zeros(P * G * 21, dtype=torch.float64, device=dev)
-        if ncol:
-            pst = post[:ncol].to(torch.float64)
-            c_t = torch.as_tensor(c_all[:ncol], device=dev)
-            a_t = torch.as_tensor(np.minimum(a_all[:ncol], 20), device=dev)
-            d_t = torch.as_tensor(np.minimum(d_all[:ncol], 20), device=dev)
-            st_t = torch.as_tensor(np.asarray(st, np.int64), device=dev)
-            gr_t = torch.as_tensor(np.asarray(gr, np.int64), device=dev)
-            for typ, out, idx_fn in ((1, cM, lambda g: (pair_of[:, None] * G + g) * 441 + a_t[:, None] * 21
-                                      + d_t[:, None]),
-                                     (2, cI, lambda g: (pair_of[:, None] * G + g) * 21 + d_t[:, None]),
-                                     (3, cD, lambda g: (pair_of[:, None] * G + g) * 21 + a_t[:, None])):
-                sel = st_t == typ
-                if not bool(sel.any()):
-                    continue
-                w = pst[:, sel] * (c_t == typ)[:, None]
-                out.index_add_(0, idx_fn(gr_t[sel][None, :]).reshape(-1), w.reshape(-1))
-        cM, cI, cD = cM.view(P, G, 21, 21), cI.view(P, G, 21), cD.view(P, G, 21)
+        cM, cI, cD = _lib.fb1d_counts(st, gr, G, lens, off, c_dev, a_dev, d_dev, post)
         ctx.save_for_backward(chi, EM, EI, ED, nt, cM, cI, cD)
         ctx.status = st1 | st2
         return ll
@@ -916,13 +895,15 @@ def mixdom2_constrained_log_prob(main_ins_rate, main_del_rate, t, dom_ins_rates,
             'classdist': classdist})
         chi = MixDom2Chi.apply(pro, tt, f(main_ins_rate), f(main_del_rate), f(dom_ins_rates), f(dom_del_rates),
                                f(dom_weights), f(frag_weights), f(ext_rates))
+        EM, EI = MixDom2Emissions.apply(pro, tt, f(class_S_exch), f(class_pis), f(classdist))
+        ED = EI
     else:
         chi = pm.build_nested_trans(f(main_ins_rate), f(main_del_rate), tt, f(dom_ins_rates),
                                     f(dom_del_rates), f(dom_weights), f(frag_weights), f(ext_rates))
-    csubs = pm.class_subs(f(class_S_exch), f(class_pis), tt)
-    EM, EI, ED = pm.tables_per_class(csubs, f(class_pis), f(classdist))
-    if EI.dim() == 2:
-        EI, ED = EI.unsqueeze(0), ED.unsqueeze(0)
+        csubs = pm.class_subs(f(class_S_exch), f(class_pis), tt)
+        EM, EI, ED = pm.tables_per_class(csubs, f(class_pis), f(classdist))
+        if EI.dim() == 2:
+            EI, ED = EI.unsqueeze(0), ED.unsqueeze(0)
     st = pm.mixdom_state_types(K, F)
     gr = pm.mixdom_state_groups(K, F)
     ll = ConstrainedLogLik.apply(chi, EM, EI, ED, st, gr, cols, ancs, descs)
@@ -1153,6 +1134,27 @@ class MixDom2Chi(torch.autograd.Function):
         return (None, *out)
 
 
+class MixDom2Emissions(torch.autograd.Function):
+    """The MixDom2 emission tables (EM [P,G,21,21], EI = ED [P,G,21], float64) built on the device
+    (phmm_mixdom2_emissions), differentiable in t, class_S_exch, class_pis and classdist through the device
+    vector-Jacobian product phmm_mixdom2_emissions_vjp (the exponential's adjoint by its Frechet derivative)."""
+
+    @staticmethod
+    def forward(ctx, pro, t, S_exch, pis, classdist):
+        tt = t.detach().to(torch.float64).reshape(-1).contiguous()
+        EM, EI, csubs = pro.emissions(tt)
+        ctx.pro = pro
+        ctx.shapes = [v.shape for v in (t, S_exch, pis, classdist)]
+        ctx.save_for_backward(tt, csubs)
+        return EM, EI
+
+    @staticmethod
+    def backward(ctx, gM, gI):
+        tt, csubs = ctx.saved_tensors
+        grads = ctx.pro.emissions_vjp(tt, csubs, gM, gI)
+        return (None, *(g.reshape(sh) for g, sh in zip(grads, ctx.shapes)))
+
+
 def mixdom2_log_prob(main_ins_rate, main_del_rate, t, dom_ins_rates, dom_del_rates, dom_weights,
                      frag_weights, ext_rates, class_pis, class_S_exch, class_dist, x_seq, y_seq):
     """log P(x, y) under MixDom2 with gradients for every tensor argument
@@ -1175,11 +1177,13 @@ def mixdom2_log_prob(main_ins_rate, main_del_rate, t, dom_ins_rates, dom_del_rat
             'classdist': class_dist})
         chi = MixDom2Chi.apply(pro, tt, f(main_ins_rate), f(main_del_rate), f(dom_ins_rates), f(dom_del_rates),
                                f(dom_weights), f(frag_weights), f(ext_rates))
+        EM, EI = MixDom2Emissions.apply(pro, tt, f(class_S_exch), f(class_pis), f(class_dist))
+        ED = EI
     else:
         chi = pm.build_nested_trans(f(main_ins_rate), f(main_del_rate), tt, f(dom_ins_rates),
                                     f(dom_del_rates), f(dom_weights), f(frag_weights), f(ext_rates))
-    csubs = pm.class_subs(f(class_S_exch), f(class_pis), tt)
-    EM, EI, ED = pm.tables_per_class(csubs, f(class_pis), f(class_dist))
+        csubs = pm.class_subs(f(class_S_exch), f(class_pis), tt)
+        EM, EI, ED = pm.tables_per_class(csubs, f(class_pis), f(class_dist))
     plan = get_plan(pm.mixdom_state_types(K, F), pm.mixdom_state_groups(K, F), K * F)
     ll = PairHMMLogLik.apply(chi, EM, EI, ED, plan, xs, ys)
     return ll if batched else ll[0]
