@@ -59,3 +59,24 @@ def test_alignment_counts(cuda_lib, n):
                 want[cols[l] - 1][at] += np.float64(post[l, s])
     for g, w in zip(got, want):
         np.testing.assert_allclose(g.cpu().numpy(), w, rtol=1e-13, atol=0)
+
+
+@pytest.mark.parametrize('K,F', [(1, 1), (2, 3), (3, 1), (4, 2), (5, 1), (8, 4), (16, 2), (33, 1)])
+def test_chi_gradients(cuda_lib, K, F):
+    """One to 33 domains: every direction at once, several rounds of teams, one team (the bound of its other test, 1e-9)."""
+    from pairhmm import _lib, api, synth
+    from pairhmm import models as pm
+    rng = np.random.default_rng(K * 10 + F)
+    p = synth.mixdom2_params(rng, K, F, 1)
+    p['ext_rates'] = rng.dirichlet(np.ones(F + 1), (K, F))[..., :F]      # a full fragment matrix
+    keys = ('main_ins', 'main_del', 'dom_ins', 'dom_del', 'dom_weights', 'frag_weights', 'ext_rates')
+    ts = np.array([0.3, 1.1])
+    leaf = lambda dev: [torch.tensor(v, dtype=torch.float64, device=dev, requires_grad=True)
+                        for v in [ts] + [p[k] for k in keys]]
+    a, b = leaf('cpu'), leaf('cuda')
+    chi = pm.build_nested_trans(a[1], a[2], a[0], *a[3:])
+    w = torch.tensor(rng.normal(size=chi.shape))
+    (chi * w).sum().backward()
+    (api.MixDom2Chi.apply(_lib.MixDom2Prologue(p), *b) * w.cuda()).sum().backward()
+    for x, y in zip(a, b):
+        assert (y.grad.cpu() - x.grad).abs().max() <= 1e-9 * x.grad.abs().max()

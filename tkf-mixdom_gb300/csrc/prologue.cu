@@ -24,6 +24,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -174,15 +175,24 @@ struct ChiParams {
     const T *dins, *ddel, *dw, *fw, *ext;
 };
 
-// Build the N x N collapsed chi of one pair (models/mixdom.py:104-423) with
-// the CTA; emit(idx, value) receives every entry (row-major, idx = r*N + c).
-template <class T, class Emit>
-__device__ void build_chi(const ChiParams<T> &cp, int K, int F, int N, ChiSmem<T> &sm, int *piv_row, Emit emit) {
-    const int tid = threadIdx.x;
+// The threads that work on one build: the whole CTA (barrier 0) or warps of it
+// that meet at a named barrier of their own.
+struct Team {
+    int tid, n, bar;
+    __device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(n) : "memory"); }
+};
+__device__ __forceinline__ Team whole_cta() { return {(int)threadIdx.x, (int)blockDim.x, 0}; }
+
+// The factors the collapsed chi of one pair is assembled from
+// (models/mixdom.py:104-252): TKF91 matrices, T_exit_k, the effective T, entry and
+// exit factors, in sm.
+template <class T>
+__device__ void build_factors(const ChiParams<T> &cp, int K, ChiSmem<T> &sm, int *piv_row, const Team &tm) {
+    const int tid = tm.tid;
     const int n3 = sm.n3, w = sm.w;
     // TKF91 matrices of the main level and of each domain level
     if (tid == 0) tkf91(cp.main_ins, cp.main_del, cp.t, sm.tau);
-    for (int k = tid; k < K; k += blockDim.x) {
+    for (int k = tid; k < K; k += tm.n) {
         tkf91(cp.dins[k], cp.ddel[k], cp.t, sm.tauK + 25 * k);
         const T kap = cp.dins[k] / cp.ddel[k];
         const T zt = (1.0 - kap) * (1.0 - tkf_beta(cp.dins[k], cp.ddel[k], cp.t));
@@ -191,7 +201,7 @@ __device__ void build_chi(const ChiParams<T> &cp, int K, int F, int N, ChiSmem<T
         sm.z[3 * k + 1] = 1.0 - kap;
         sm.z[3 * k + 2] = 1.0 - kap;
     }
-    __syncthreads();
+    tm.sync();
 
     // null-domain quantities (models/mixdom.py:104-214): for flat index
     // i = 3k + e (e over the M, I, D contexts), z(i) is the probability that
@@ -199,7 +209,7 @@ __device__ void build_chi(const ChiParams<T> &cp, int K, int F, int N, ChiSmem<T
     const T *tau = sm.tau;
     const T tauE[3] = {tau[M * 5 + E], tau[M * 5 + E], tau[D * 5 + E]};
     const int nullrow[3] = {M, M, D};
-    for (int i = tid; i < n3; i += blockDim.x) {
+    for (int i = tid; i < n3; i += tm.n) {
         const int k = i / 3, e = i % 3;
         const T z = sm.z[i];
         const T nonnull = e == 0 ? 1.0 - z : sm.kap[k];
@@ -213,7 +223,7 @@ __device__ void build_chi(const ChiParams<T> &cp, int K, int F, int N, ChiSmem<T
         // right-hand sides: T_Nnull[u][i] = tau[u][MID[e]] dw[k]
         for (int u = 0; u < 5; ++u) sm.aug[i * w + n3 + u] = tau[u * 5 + MID[e]] * cp.dw[k];
     }
-    __syncthreads();
+    tm.sync();
 
     // Gauss-Jordan with partial pivoting: (I - T_nn)^T Y^T = T_Nnull^T
     for (int c = 0; c < n3; ++c) {
@@ -226,39 +236,39 @@ __device__ void build_chi(const ChiParams<T> &cp, int K, int F, int N, ChiSmem<T
             }
             *piv_row = best;
         }
-        __syncthreads();
+        tm.sync();
         const int pr = *piv_row;
         if (pr != c)
-            for (int j = tid; j < w; j += blockDim.x) {
+            for (int j = tid; j < w; j += tm.n) {
                 const T a = sm.aug[c * w + j];
                 sm.aug[c * w + j] = sm.aug[pr * w + j];
                 sm.aug[pr * w + j] = a;
             }
-        __syncthreads();
+        tm.sync();
         const T inv = 1.0 / sm.aug[c * w + c];
-        __syncthreads();
-        for (int j = tid; j < w; j += blockDim.x) sm.aug[c * w + j] = sm.aug[c * w + j] * inv;
-        __syncthreads();
-        for (int idx = tid; idx < n3 * w; idx += blockDim.x) {
+        tm.sync();
+        for (int j = tid; j < w; j += tm.n) sm.aug[c * w + j] = sm.aug[c * w + j] * inv;
+        tm.sync();
+        for (int idx = tid; idx < n3 * w; idx += tm.n) {
             const int r = idx / w, j = idx % w;
             if (r == c || j == c) continue;
             sm.aug[idx] = sm.aug[idx] - sm.aug[r * w + c] * sm.aug[c * w + j];
         }
-        __syncthreads();
-        for (int r = tid; r < n3; r += blockDim.x)
+        tm.sync();
+        for (int r = tid; r < n3; r += tm.n)
             if (r != c) sm.aug[r * w + c] = cst<T>(0.0);
-        __syncthreads();
+        tm.sync();
     }
 
     // T_exit_k[k][u][v] = sum_e Y[u][3k+e] T_nullN[3k+e][v]; Y[u][i] = aug[i][3K+u]
-    for (int idx = tid; idx < 25 * K; idx += blockDim.x) {
+    for (int idx = tid; idx < 25 * K; idx += tm.n) {
         const int k = idx / 25, u = (idx / 5) % 5, v = idx % 5;
         T s = cst<T>(0.0);
         for (int e = 0; e < 3; ++e) s = s + sm.aug[(3 * k + e) * w + n3 + u] * sm.TnN[(3 * k + e) * 5 + v];
         sm.Tex[idx] = s;
     }
     // entry / exit factors of each domain's five sub-states
-    for (int idx = tid; idx < 5 * K; idx += blockDim.x) {
+    for (int idx = tid; idx < 5 * K; idx += tm.n) {
         const int k = idx / 5, j = idx % 5;
         const T *tk = sm.tauK + 25 * k;
         const T beta_d = floor_at(1.0 - tk[S * 5 + E], 1e-30);
@@ -266,13 +276,21 @@ __device__ void build_chi(const ChiParams<T> &cp, int K, int F, int N, ChiSmem<T
         sm.ent[idx] = isM ? tk[S * 5 + UV_X[j]] / beta_d : cst<T>(1.0);
         sm.exi[idx] = isM ? tk[UV_X[j] * 5 + E] : 1.0 - sm.kap[k];
     }
-    __syncthreads();
-    for (int idx = tid; idx < 25; idx += blockDim.x) {
+    tm.sync();
+    for (int idx = tid; idx < 25; idx += tm.n) {
         T s = (idx % 5 == E) ? tau[idx] : cst<T>(0.0);
         for (int k = 0; k < K; ++k) s = s + sm.Tex[25 * k + idx];
         sm.T5[idx] = s;
     }
-    __syncthreads();
+    tm.sync();
+}
+
+// Build the N x N collapsed chi of one pair (models/mixdom.py:104-423) with
+// the CTA; emit(idx, value) receives every entry (row-major, idx = r*N + c).
+template <class T, class Emit>
+__device__ void build_chi(const ChiParams<T> &cp, int K, int F, int N, ChiSmem<T> &sm, int *piv_row, Emit emit) {
+    const int tid = threadIdx.x;
+    build_factors(cp, K, sm, piv_row, whole_cta());
 
     // chi (models/mixdom.py:252-423): state 0 = SS, 1 = EE, body state
     // 2 + k*5F + j*F + f (domain k, sub-state j, fragment f)
@@ -394,38 +412,186 @@ chi_kernel_dp(const Packed *__restrict__ prm, const double *__restrict__ ts, int
     chi_kernel_body(*prm, ts, N, chi, chi64, nest);
 }
 
-// Vector-Jacobian product of chi: for pair p = blockIdx.x and parameter
-// direction d = blockIdx.y, grad[p][d] = sum_{s,k} G[p][s][k] dchi[s][k]/dtheta_d,
-// by one forward-mode (Dual) pass of the builder seeded on theta_d.
-// Directions: 0 main_ins, 1 main_del, 2 t, 3 + j the j-th entry of the packed
-// domain arrays (dom_ins[K], dom_del[K], dom_w[K], frag_w[K*F], ext[K*F*F]).
-__global__ void __launch_bounds__(THREADS)
-chi_vjp_kernel(const __grid_constant__ Packed prm, const double *__restrict__ ts, int N,
-               const double *__restrict__ G, double *__restrict__ grad) {
-    extern __shared__ Dual smem_dual[];
-    __shared__ int piv_row;
-    __shared__ double red[THREADS / 32];
-    const int p = blockIdx.x, dir = blockIdx.y, nd = gridDim.y, tid = threadIdx.x;
-    const int K = prm.K, F = prm.F;
-    const int nparam = 3 * K + K * F + K * F * F;
-    ChiSmem<Dual> sm;
-    sm.carve(smem_dual, K);
-    Dual *pv = smem_dual + ChiSmem<Dual>::elems(K);   // the packed domain arrays as Duals
-    for (int j = tid; j < nparam; j += blockDim.x) pv[j] = mkd(prm.v[prm.o_dins + j], dir == 3 + j ? 1.0 : 0.0);
-    __syncthreads();
-    const ChiParams<Dual> cp{mkd(prm.main_ins, dir == 0 ? 1.0 : 0.0), mkd(prm.main_del, dir == 1 ? 1.0 : 0.0),
-                             mkd(ts[p], dir == 2 ? 1.0 : 0.0), pv, pv + K, pv + 2 * K, pv + 3 * K,
-                             pv + 3 * K + K * F};
+// Vector-Jacobian product of chi: grad[p][d] = sum_{s,k} G[p][s][k]
+// dchi[s][k]/dtheta_d for pair p = blockIdx.x and every parameter direction d: 0
+// main_ins, 1 main_del, 2 t, 3 + j the j-th entry of the packed domain arrays
+// (dom_ins[K], dom_del[K], dom_w[K], frag_w[K*F], ext[K*F*F]).
+//
+// chi is assembled from few factors, so G is contracted with the assembly once, in
+// reverse, to the factors' adjoints (T_exit_k, T, entry, exit, the domains' TKF91
+// matrices and kappas, frag_w and ext); those of frag_w and ext are already their
+// gradients, and each remaining direction (3 + 3 K) is one forward-mode (Dual) pass
+// of build_factors by a team of warps, dotted with the adjoints.  FP64 bounds it.
+// One CTA per pair and direction, each a Dual pass over all N^2 entries, took 0.81
+// ms for 64 pairs at 42 states (39 directions), now 0.29.
+struct ChiAdjoint {   // doubles, after the teams' workspaces
+    double *Tex, *T5, *ent, *exi, *tauK, *kap, *fw, *ext, *X, *D, *gX, *gD, *nx;
+    __device__ void carve(double *p, int K, int F) {
+        Tex = p;            // [K][25]
+        T5 = Tex + 25 * K;  // [25]
+        ent = T5 + 25;      // [K][5]
+        exi = ent + 5 * K;  // [K][5]
+        tauK = exi + 5 * K; // [K][25]
+        kap = tauK + 25 * K;
+        fw = kap + K;       // [K][F]
+        ext = fw + K * F;   // [K][F][F]
+        X = ext + K * F * F;    // [5KF] exit factors, D entry factors, and their adjoints
+        D = X + 5 * K * F;
+        gX = D + 5 * K * F;
+        gD = gX + 5 * K * F;
+        nx = gD + 5 * K * F;    // [KF] 1 - the fragment's extensions
+    }
+    __host__ __device__ static size_t elems(int K, int F) {
+        return 61 * (size_t)K + 25 + 22 * (size_t)K * F + (size_t)K * F * F;
+    }
+};
+
+__global__ void __launch_bounds__(512)
+chi_vjp_kernel(const __grid_constant__ Packed prm, const double *__restrict__ ts, int N, const double *__restrict__ G,
+               double *__restrict__ grad, int teams, int team_threads) {
+    extern __shared__ __align__(16) double vjp_smem[];
+    __shared__ int piv_row[16];
+    const int p = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
+    const int K = prm.K, F = prm.F, KF = K * F, nd = 3 + 3 * K + KF + KF * F, nb = 5 * KF, bs = 5 * F;
     const double *Gp = G + (size_t)p * N * N;
-    double acc = 0.0;
-    build_chi(cp, K, F, N, sm, &piv_row, [&](int idx, Dual v) { acc += Gp[idx] * v.d; });
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((tid & 31) == 0) red[tid >> 5] = acc;
+    const double *fw = prm.v + prm.o_fw, *ext = prm.v + prm.o_ext;
+    const size_t team_duals = ChiSmem<Dual>::elems(K) + 3 * K;
+    ChiAdjoint ad;
+    ad.carve(vjp_smem + 2 * team_duals * teams, K, F);
+    // values: the factors, in the first team's workspace
+    ChiSmem<double> sm;
+    sm.carve(vjp_smem, K);
+    {
+        const ChiParams<double> cp{prm.main_ins, prm.main_del, ts[p], prm.v + prm.o_dins, prm.v + prm.o_ddel,
+                                   prm.v + prm.o_dw, fw, ext};
+        build_factors(cp, K, sm, piv_row, whole_cta());
+    }
+    for (int i = tid; i < (int)(ad.X - ad.Tex); i += nt) ad.Tex[i] = 0.0;
+    for (int q = tid; q < KF; q += nt) {
+        double x = 1.0;
+        for (int g = 0; g < F; ++g) x -= ext[q * F + g];
+        ad.nx[q] = x;
+    }
     __syncthreads();
-    if (tid == 0) {
-        double s = 0.0;
-        for (int i = 0; i < (int)(blockDim.x >> 5); ++i) s += red[i];
-        grad[(size_t)p * nd + dir] = s;
+    for (int q = tid; q < nb; q += nt) {
+        const int k = q / bs, j = (q % bs) / F, kf = k * F + q % F;
+        ad.X[q] = ad.nx[kf] * sm.exi[5 * k + j];
+        ad.D[q] = fw[kf] * sm.ent[5 * k + j];
+    }
+    __syncthreads();
+    // a warp per sum over a row or column of G
+    const int lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
+    auto warp_sum = [](double v) {
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        return v;
+    };
+    for (int job = warp; job < 2 * nb + 12 * K + 4; job += nw) {
+        double x = 0.0;
+        if (job < nb) {                         // exit factor of source r
+            const int r = job, U = UV_U[(r % bs) / F];
+            const double *g = Gp + (size_t)(2 + r) * N;
+            for (int c = lane; c < nb; c += 32) x += g[2 + c] * (sm.Tex[25 * (c / bs) + U * 5 + UV_U[(c % bs) / F]] * ad.D[c]);
+            x = warp_sum(x);
+            if (lane == 0) ad.gX[r] = x + g[1] * sm.T5[U * 5 + E];
+        } else if (job < 2 * nb) {              // entry factor of destination c
+            const int c = job - nb, k = c / bs, U = UV_U[(c % bs) / F];
+            for (int r = lane; r < nb; r += 32)
+                x += Gp[(size_t)(2 + r) * N + 2 + c] * (ad.X[r] * sm.Tex[25 * k + UV_U[(r % bs) / F] * 5 + U]);
+            x = warp_sum(x);
+            if (lane == 0) ad.gD[c] = x + Gp[2 + c] * sm.Tex[25 * k + S * 5 + U];
+        } else if (job < 2 * nb + 12 * K) {     // T_exit_k between top-level types u = S, M, I, D and v = M, I, D
+            const int q = job - 2 * nb, k = q / 12, u = (q / 3) % 4, v = MID[q % 3];
+            for (int cj = 0; cj < bs; ++cj) {
+                if (UV_U[cj / F] != v) continue;
+                const int c = k * bs + cj;
+                double y = 0.0;
+                if (u == S) y = lane == 0 ? Gp[2 + c] : 0.0;
+                else
+                    for (int r = lane; r < nb; r += 32)
+                        if (UV_U[(r % bs) / F] == u) y += Gp[(size_t)(2 + r) * N + 2 + c] * ad.X[r];
+                x += y * ad.D[c];
+            }
+            x = warp_sum(x);
+            if (lane == 0) ad.Tex[25 * k + u * 5 + v] = x;
+        } else {                                // T to the end
+            const int u = job - 2 * nb - 12 * K;
+            if (u == S) x = lane == 0 ? Gp[1] : 0.0;
+            else
+                for (int r = lane; r < nb; r += 32)
+                    if (UV_U[(r % bs) / F] == u) x += Gp[(size_t)(2 + r) * N + 1] * ad.X[r];
+            x = warp_sum(x);
+            if (lane == 0) ad.T5[u * 5 + E] = x;
+        }
+    }
+    __syncthreads();
+    // the factors within a domain: few terms each (G of the same-domain block: gb(k, j f, j' f'))
+    auto gb = [&](int k, int jf, int jq) { return Gp[(size_t)(2 + k * bs + jf) * N + 2 + k * bs + jq]; };
+    for (int job = tid; job < 10 * K + 9 * K + K + 2 * KF; job += nt) {
+        double x = 0.0;
+        if (job < 10 * K) {                     // exit and entry factors of a sub-state
+            const int q = job % (5 * K), k = q / 5, j = q % 5;
+            for (int f = 0; f < F; ++f)
+                x += job < 5 * K ? ad.gX[k * bs + j * F + f] * ad.nx[k * F + f] : ad.gD[k * bs + j * F + f] * fw[k * F + f];
+            (job < 5 * K ? ad.exi : ad.ent)[q] = x;
+        } else if (job < 19 * K) {              // the domain's TKF91 matrix between M, I, D
+            const int q = job - 10 * K, k = q / 9, j = (q / 3) % 3, jq = q % 3;
+            for (int f = 0; f < F; ++f)
+                for (int h = 0; h < F; ++h) x += gb(k, j * F + f, jq * F + h) * (ad.nx[k * F + f] * fw[k * F + h]);
+            ad.tauK[25 * k + MID[j] * 5 + MID[jq]] = x;
+        } else if (job < 20 * K) {
+            const int k = job - 19 * K;
+            for (int j = 3; j < 5; ++j)
+                for (int f = 0; f < F; ++f)
+                    for (int h = 0; h < F; ++h) x += gb(k, j * F + f, j * F + h) * (ad.nx[k * F + f] * fw[k * F + h]);
+            ad.kap[k] = x;
+        } else {                                // a fragment's weight (as destination) or its extensions (as source)
+            const bool weight = job < 20 * K + KF;
+            const int q = (job - 20 * K) % KF, k = q / F, f = q % F;
+            for (int j = 0; j < 5; ++j)
+                for (int jq = j < 3 ? 0 : j; jq < (j < 3 ? 3 : j + 1); ++jq) {
+                    const double m = j < 3 ? sm.tauK[25 * k + MID[j] * 5 + MID[jq]] : sm.kap[k];
+                    for (int h = 0; h < F; ++h)
+                        x += weight ? gb(k, j * F + h, jq * F + f) * (ad.nx[k * F + h] * m)
+                                    : gb(k, j * F + f, jq * F + h) * (m * fw[k * F + h]);
+                }
+            for (int j = 0; j < 5; ++j)
+                x += weight ? ad.gD[k * bs + j * F + f] * sm.ent[5 * k + j] : ad.gX[k * bs + j * F + f] * sm.exi[5 * k + j];
+            if (weight) {
+                ad.fw[q] = x;
+            } else {
+                for (int h = 0; h < F; ++h) {
+                    double e = -x;
+                    for (int j = 0; j < 5; ++j) e += gb(k, j * F + f, j * F + h);
+                    ad.ext[q * F + h] = e;
+                }
+            }
+        }
+    }
+    __syncthreads();
+    for (int i = tid; i < KF + KF * F; i += nt) grad[(size_t)p * nd + 3 + 3 * K + i] = ad.fw[i];   // ext follows fw
+    // the other directions, one team of warps each
+    const int team = tid / team_threads;
+    const Team tm{tid % team_threads, team_threads, 1 + team};
+    ChiSmem<Dual> ds;
+    Dual *base = reinterpret_cast<Dual *>(vjp_smem) + team_duals * team;
+    ds.carve(base, K);
+    Dual *pv = base + ChiSmem<Dual>::elems(K);
+    for (int dir = team; dir < 3 + 3 * K; dir += teams) {
+        tm.sync();
+        for (int j = tm.tid; j < 3 * K; j += tm.n) pv[j] = mkd(prm.v[prm.o_dins + j], dir == 3 + j ? 1.0 : 0.0);
+        tm.sync();
+        const ChiParams<Dual> cp{mkd(prm.main_ins, dir == 0 ? 1.0 : 0.0), mkd(prm.main_del, dir == 1 ? 1.0 : 0.0),
+                                 mkd(ts[p], dir == 2 ? 1.0 : 0.0), pv, pv + K, pv + 2 * K, nullptr, nullptr};
+        build_factors(cp, K, ds, &piv_row[team], tm);
+        if (tm.tid < 32) {
+            double acc = 0.0;
+            for (int i = tm.tid; i < 25 * K; i += 32) acc += ad.Tex[i] * ds.Tex[i].d + ad.tauK[i] * ds.tauK[i].d;
+            for (int i = tm.tid; i < 5 * K; i += 32) acc += ad.ent[i] * ds.ent[i].d + ad.exi[i] * ds.exi[i].d;
+            for (int i = tm.tid; i < K; i += 32) acc += ad.kap[i] * ds.kap[i].d;
+            if (tm.tid < 25) acc += ad.T5[tm.tid] * ds.T5[tm.tid].d;
+            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+            if (tm.tid == 0) grad[(size_t)p * nd + dir] = acc;
+        }
     }
 }
 
@@ -1284,14 +1450,22 @@ extern "C" int phmm_mixdom2_chi_vjp(const phmm_mixdom2_params *prm, int32_t n_pa
     if (!t || !grad_chi || !grad) return pro_fail(PHMM_E_ARG, "phmm_mixdom2_chi_vjp: null device buffer");
     const int K = pk.K, F = pk.F;
     const int N = 2 + 5 * K * F;
-    const int nd = 3 + 3 * K + K * F + K * F * F;
-    const size_t smem = sizeof(Dual) * (ChiSmem<Dual>::elems(K) + (size_t)(nd - 3));
-    if (smem > 227 * 1024) return pro_fail(PHMM_E_ARG, "phmm_mixdom2_chi_vjp: state space too large");
+    // as many directions at a time as shared memory and 15 named barriers allow, a warp or more each
+    const size_t per_team = sizeof(Dual) * (ChiSmem<Dual>::elems(K) + 3 * (size_t)K);
+    const size_t fixed = sizeof(double) * ChiAdjoint::elems(K, F);
+    if (per_team + fixed > 227 * 1024) return pro_fail(PHMM_E_ARG, "phmm_mixdom2_chi_vjp: state space too large");
+    const int dirs = 3 + 3 * K;
+    int teams = (int)std::min<size_t>(std::min(15, dirs), (227 * 1024 - 1024 - fixed) / per_team);
+    if (teams < 1) teams = 1;
+    teams = (dirs + (dirs + teams - 1) / teams - 1) / ((dirs + teams - 1) / teams);   // even rounds
+    const int team_threads = std::max(32, 512 / teams / 32 * 32);
+    const size_t smem = per_team * teams + fixed;
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(chi_vjp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return pro_fail(PHMM_E_CUDA, cudaGetErrorString(e));
     }
-    chi_vjp_kernel<<<dim3(n_pairs, nd), THREADS, smem, (cudaStream_t)stream>>>(pk, t, N, grad_chi, grad);
+    chi_vjp_kernel<<<n_pairs, teams * team_threads, smem, (cudaStream_t)stream>>>(pk, t, N, grad_chi, grad, teams,
+                                                                                 team_threads);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return pro_fail(PHMM_E_CUDA, cudaGetErrorString(e));
     return PHMM_OK;
