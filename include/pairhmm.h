@@ -465,6 +465,13 @@ int phmm_pairs_decode(const char *text, size_t len, const phmm_pair_counts *size
                       int64_t *col_off, int8_t *col_state, uint8_t *col_anc, uint8_t *col_desc,
                       int64_t *fam_off, int32_t *fam_len);
 
+/* Padded batches (the reference's xs_pad / ys_pad, train/tkf92_svi_bw.py:263-334)
+ * into phmm_batch's residue layout, on the host: rows of x_width / y_width integers
+ * of item_bytes (1, 2, 4, 8), pair p's first Lx[p] of x and Ly[p] of y written one
+ * after the other.  PHMM_E_ARG when a residue lies outside 0..20. */
+int phmm_pack_padded(int32_t n_pairs, const void *x, int64_t x_width, const void *y, int64_t y_width,
+                     int32_t item_bytes, int32_t is_signed, const int32_t *Lx, const int32_t *Ly, uint8_t *residues);
+
 /* TKF91 / TKF92 parameters (host float64): insertion and deletion rates,
  * fragment extension probability (0 for TKF91), the substitution rate
  * matrix Q [A][A] (rows summing to zero) and its equilibrium pi [A]; A = 20. */

@@ -370,3 +370,57 @@ extern "C" int phmm_pairs_decode(const char *text, size_t len, const phmm_pair_c
     }
     return PHMM_OK;
 }
+
+namespace {
+
+// One padded batch of T residues; false at a residue outside 0..20.
+template <class T>
+bool pack_rows(int32_t n, const T *x, int64_t xw, const T *y, int64_t yw, const int32_t *Lx, const int32_t *Ly, uint8_t *out) {
+    bool ok = true;
+    auto row = [&](const T *r, int32_t len) {
+        for (int32_t i = 0; i < len; ++i) {
+            ok &= r[i] >= T(0) && r[i] <= T(20);
+            out[i] = (uint8_t)r[i];
+        }
+        out += len;
+    };
+    for (int32_t p = 0; p < n; ++p) {
+        row(x + p * xw, Lx[p]);
+        row(y + p * yw, Ly[p]);
+    }
+    return ok;
+}
+
+}  // namespace
+
+extern "C" int phmm_pack_padded(int32_t n_pairs, const void *x, int64_t x_width, const void *y, int64_t y_width,
+                                int32_t item_bytes, int32_t is_signed, const int32_t *Lx, const int32_t *Ly,
+                                uint8_t *residues) {
+    if (n_pairs < 0) { phmm_internal_set_error("phmm_pack_padded: negative n_pairs"); return PHMM_E_ARG; }
+    if (n_pairs == 0) return PHMM_OK;
+    if (!x || !y || !Lx || !Ly || !residues) {
+        phmm_internal_set_error("phmm_pack_padded: null pointer");
+        return PHMM_E_ARG;
+    }
+    for (int32_t p = 0; p < n_pairs; ++p)
+        if (Lx[p] < 0 || Lx[p] > x_width || Ly[p] < 0 || Ly[p] > y_width) {
+            phmm_internal_set_error("phmm_pack_padded: length outside its row");
+            return PHMM_E_ARG;
+        }
+    bool ok = false;
+#define PACK(T) ok = pack_rows(n_pairs, (const T *)x, x_width, (const T *)y, y_width, Lx, Ly, residues)
+    switch (item_bytes * 2 + (is_signed ? 1 : 0)) {
+        case 2: PACK(uint8_t); break;
+        case 3: PACK(int8_t); break;
+        case 4: PACK(uint16_t); break;
+        case 5: PACK(int16_t); break;
+        case 8: PACK(uint32_t); break;
+        case 9: PACK(int32_t); break;
+        case 16: PACK(uint64_t); break;
+        case 17: PACK(int64_t); break;
+        default: phmm_internal_set_error("phmm_pack_padded: integers of 1, 2, 4 or 8 bytes"); return PHMM_E_ARG;
+    }
+#undef PACK
+    if (!ok) phmm_internal_set_error("phmm_pack_padded: residues must be in 0..20");
+    return ok ? PHMM_OK : PHMM_E_ARG;
+}

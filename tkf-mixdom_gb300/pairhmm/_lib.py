@@ -32,7 +32,7 @@ EXPORTS = ('phmm_plan_create', 'phmm_plan_destroy', 'phmm_forward', 'phmm_estep'
            'phmm_mixdom2_param_block', 'phmm_mixdom2_tables_dp', 'phmm_mixdom2_class_counts_dp',
            'phmm_holmes_rubin_block_bytes', 'phmm_holmes_rubin_block', 'phmm_holmes_rubin_dp',
            'phmm_mixdom2_nest', 'phmm_mixdom2_nest_dp', 'phmm_nest_supported', 'phmm_mixdom2_tables_nest',
-           'phmm_mixdom2_tables_nest_dp')
+           'phmm_mixdom2_tables_nest_dp', 'phmm_pack_padded')
 
 
 class Tuning(ctypes.Structure):
@@ -160,6 +160,8 @@ def load(path=None):
     lib.phmm_mixdom2_chi_vjp.restype = ctypes.c_int
     lib.phmm_tkf92_tables.argtypes = [ctypes.POINTER(Tkf92Params), ctypes.c_int32] + [vp] * 7
     lib.phmm_tkf92_tables.restype = ctypes.c_int
+    lib.phmm_pack_padded.argtypes = [i32, vp, i64, vp, i64, i32, i32, ctypes.POINTER(i32), ctypes.POINTER(i32), vp]
+    lib.phmm_pack_padded.restype = ctypes.c_int
     lib.phmm_mixdom2_emissions.argtypes = [ctypes.POINTER(MixDom2Params), ctypes.c_int32] + [vp] * 5
     lib.phmm_mixdom2_emissions.restype = ctypes.c_int
     lib.phmm_mixdom2_emissions_vjp_work.argtypes = [ctypes.POINTER(MixDom2Params), ctypes.c_int32]
@@ -369,6 +371,36 @@ class DeviceBatch:
         return self._struct
 
 
+# host arrays up to _UPLOAD_INLINE bytes go into the launch stream itself (CUDA takes a host-to-device copy of 64 KB
+# or less before the call returns); above _UPLOAD_MAX their staging would cost more than the wait it saves
+_UPLOAD_INLINE, _UPLOAD_MAX = 1 << 16, 1 << 20
+
+
+def upload(a, device, dtype=None):
+    """A host array as a device tensor (of `dtype`), its values as they are now, without waiting for the work already
+    on the stream: a plain copy from pageable memory does, and a batched call's host part then starts over behind the
+    previous call's kernels.  Larger arrays go through pinned memory of torch's caching host allocator."""
+    a = np.asarray(a)
+    src = torch.from_numpy(a) if a.flags.writeable else torch.as_tensor(a)
+    dt = src.dtype if dtype is None else dtype
+    nb = src.numel() * _ESIZE.get(dt, 8)
+    if torch.device(device).type != 'cuda' or nb > _UPLOAD_MAX:
+        return src.to(device=device, dtype=dt).contiguous()
+    if nb <= _UPLOAD_INLINE:
+        host = torch.empty(src.shape, dtype=dt)   # (the caller's own memory may be pinned, and then copied late)
+    else:
+        host = torch.empty(src.shape, dtype=dt, pin_memory=True)
+    host.copy_(src)
+    return host.to(device, non_blocking=True)
+
+
+def concat_u8(arrays):
+    """The arrays' elements one after the other as uint8."""
+    if all(type(v) is np.ndarray and v.ndim == 1 for v in arrays) and len(arrays):
+        return np.concatenate(arrays, dtype=np.uint8, casting='unsafe')
+    return np.concatenate([np.asarray(v, np.uint8).reshape(-1) for v in arrays])
+
+
 def pack_residues(xs, ys):
     """Concatenate residues of all pairs: [x_0, y_0, x_1, y_1, ...] (uint8)."""
     P = len(xs)
@@ -493,19 +525,46 @@ class OutputArena:
         return self.t[name]
 
 
+def pack_padded(x_pad, y_pad, Lx, Ly):
+    """pack_residues of padded integer arrays [P, width] cut to their lengths, natively; None where the arrays or
+    lengths are of another form (the caller then cuts them one by one)."""
+    ok = lambda m, L: (type(m) is np.ndarray and m.ndim == 2 and m.flags.c_contiguous and m.dtype.isnative
+                       and m.dtype.kind in 'iu' and m.shape[0] == L.size)
+    Lx, Ly = np.asarray(Lx), np.asarray(Ly)
+    if Lx.dtype.kind not in 'iu' or Ly.dtype.kind not in 'iu' or Lx.ndim != 1 or Lx.shape != Ly.shape or Lx.size == 0:
+        return None
+    if not (ok(x_pad, Lx) and ok(y_pad, Ly) and x_pad.dtype == y_pad.dtype):
+        return None
+    if Lx.min() < 0 or Ly.min() < 0 or Lx.max() > x_pad.shape[1] or Ly.max() > y_pad.shape[1]:
+        return None
+    Lx, Ly = Lx.astype(np.int32), Ly.astype(np.int32)
+    ends = np.cumsum(np.stack([Lx, Ly], axis=1).reshape(-1), dtype=np.int64)
+    xo, yo = np.concatenate([[0], ends[1:-1:2]]), ends[0::2]
+    buf = np.zeros(max(int(ends[-1]), 16 if ends[-1] == 0 else 0), np.uint8)
+    i32p, i64p = ctypes.POINTER(ctypes.c_int32), ctypes.POINTER(ctypes.c_int64)
+    rc = load().phmm_pack_padded(Lx.size, x_pad.ctypes.data, x_pad.shape[1], y_pad.ctypes.data, y_pad.shape[1],
+                                 x_pad.dtype.itemsize, int(x_pad.dtype.kind == 'i'), Lx.ctypes.data_as(i32p),
+                                 Ly.ctypes.data_as(i32p), buf.ctypes.data)
+    if rc:
+        raise ValueError('residues must be integers in 0..20 (20 = wildcard)')
+    return buf, np.ascontiguousarray(xo, np.int64), np.ascontiguousarray(yo), Lx, Ly
+
+
 def make_batch(xs, ys, chi, emit_M, emit_I, emit_D, device='cuda', cell_masks=None, beam_log_width=0.0,
-               nest=None, nest_kf=None):
+               nest=None, nest_kf=None, packed=None):
     """Build a DeviceBatch from host sequences and float tables.
 
     chi: [P or 1, N, N]; emit_*: [P or 1, G, ...] (numpy or torch, any float);
     cell_masks: optional list of per-pair uint8 arrays (Lx+1, Ly+1) (bit 0 M,
     1 I, 2 D may emit at the cell); nest: optional [P or 1, R] factored
-    MixDom transitions of chi (models.nested_record) with nest_kf = (K, F)."""
-    buf, xo, yo, Lx, Ly = pack_residues(xs, ys)
+    MixDom transitions of chi (models.nested_record) with nest_kf = (K, F);
+    packed: the sequences as pack_residues returns them, instead of xs, ys."""
+    buf, xo, yo, Lx, Ly = pack_residues(xs, ys) if packed is None else packed
 
     def dev(a, dt):
-        t = torch.as_tensor(np.asarray(a) if not isinstance(a, torch.Tensor) else a)
-        return t.to(device=device, dtype=dt).contiguous()
+        if not isinstance(a, torch.Tensor):
+            return upload(a, device, dt)
+        return a.to(device=device, dtype=dt).contiguous()
     cm = None
     if cell_masks is not None:
         if len(cell_masks) != Lx.size:
@@ -647,7 +706,7 @@ def estep_band(plan, batch, band_centers, band_half_width, stream=None):
     centers = np.concatenate([np.asarray(c, np.int32)[:int(a) + 1] for c, a in zip(band_centers, batch.Lx)])
     if centers.size != int((batch.Lx.astype(np.int64) + 1).sum()):
         raise ValueError('band_centers: Lx+1 centre columns per pair')
-    d_centers = torch.as_tensor(centers).to(dev)
+    d_centers = upload(centers, dev)
     out = {
         'll': torch.empty(P, dtype=torch.float64, device=dev),
         'n_trans': torch.empty(P, N, N, dtype=torch.float64, device=dev),
@@ -666,6 +725,20 @@ def estep_band(plan, batch, band_centers, band_half_width, stream=None):
     return out
 
 
+def _host_params(params, keys):
+    """params with the device tensors among `keys` as host float64 arrays, brought over in one copy."""
+    on_dev = [k for k in keys if isinstance(params[k], torch.Tensor) and params[k].is_cuda]
+    if len(on_dev) < 2 or len({params[k].device for k in on_dev}) > 1:
+        return params
+    flat = [params[k].detach().to(torch.float64).reshape(-1) for k in on_dev]
+    all_ = torch.cat(flat).cpu().numpy()
+    out, o = dict(params), 0
+    for k, v in zip(on_dev, flat):
+        out[k] = all_[o:o + v.numel()].reshape(tuple(params[k].shape))
+        o += v.numel()
+    return out
+
+
 class MixDom2Prologue:
     """phmm_mixdom2_tables for one MixDom2 parameter set: packs the host
     parameter arrays once, then builds the E-step inputs of any batch of
@@ -680,6 +753,7 @@ class MixDom2Prologue:
 
     def __init__(self, params):
         self.lib = load()
+        params = _host_params(params, self.KEYS + ('main_ins', 'main_del'))
         host = lambda v: v.detach().cpu().numpy() if isinstance(v, torch.Tensor) else v
         arr = {k: np.ascontiguousarray(np.asarray(host(params[k]), dtype=np.float64)) for k in self.KEYS}
         self.K = arr['dom_ins'].size
@@ -814,7 +888,7 @@ class MixDom2Prologue:
         if isinstance(ts, torch.Tensor):
             t = ts.to(device=device, dtype=torch.float64).reshape(-1).contiguous()
         else:
-            t = torch.from_numpy(np.ascontiguousarray(np.asarray(ts, np.float64).reshape(-1))).to(device)
+            t = upload(np.asarray(ts, np.float64).reshape(-1), device)
         shp = self.shapes(t.numel())
         f32, f64 = torch.float32, torch.float64
         outs = [torch.empty(sh, dtype=f64 if i == 4 else f32, device=t.device) for i, sh in enumerate(shp)]
@@ -863,7 +937,7 @@ class Tkf92Prologue:
         if isinstance(ts, torch.Tensor):
             t = ts.to(device=device, dtype=torch.float64).reshape(-1).contiguous()
         else:
-            t = torch.from_numpy(np.ascontiguousarray(np.asarray(ts, np.float64).reshape(-1))).to(device)
+            t = upload(np.asarray(ts, np.float64).reshape(-1), device)
         shp = self.shapes(t.numel())
         outs = [torch.empty(sh, dtype=torch.float64 if i == 4 else torch.float32, device=t.device)
                 for i, sh in enumerate(shp)]
@@ -902,12 +976,12 @@ def sample_paths(state_types, groups, G, xs, ys, log_chi, log_M, log_I, log_D, n
                    gr.ctypes.data_as(ctypes.POINTER(ctypes.c_int32)), int(G))
     buf, xo, yo, Lx, Ly = pack_residues(xs, ys)
     P, S = Lx.size, int(n_samples)
-    f64 = lambda a: (a if isinstance(a, torch.Tensor) else torch.as_tensor(np.asarray(a))).to(
-        device=device, dtype=torch.float64).contiguous()
+    f64 = lambda a: (a.to(device=device, dtype=torch.float64).contiguous() if isinstance(a, torch.Tensor)
+                     else upload(a, device, torch.float64))
     lc, lm, li, ld = f64(log_chi), f64(log_M), f64(log_I), f64(log_D)
     if lc.dim() == 2:
         lc = lc.unsqueeze(0)
-    res_t = torch.from_numpy(buf).to(device)
+    res_t = upload(buf, device)
     b = DeviceBatch(Lx=Lx, Ly=Ly, x_off=xo, y_off=yo, residues=res_t, chi=lc, emit_M=lm, emit_I=li, emit_D=ld)
     bs = b.struct()
     nb = ctypes.c_size_t(0)
@@ -1046,12 +1120,12 @@ def viterbi(state_types, groups, G, xs, ys, log_chi, log_M, log_I, log_D, device
                    gr.ctypes.data_as(ctypes.POINTER(ctypes.c_int32)), int(G))
     buf, xo, yo, Lx, Ly = pack_residues(xs, ys)
     P = Lx.size
-    f64 = lambda a: (a if isinstance(a, torch.Tensor) else torch.as_tensor(np.asarray(a))).to(
-        device=device, dtype=torch.float64).contiguous()
+    f64 = lambda a: (a.to(device=device, dtype=torch.float64).contiguous() if isinstance(a, torch.Tensor)
+                     else upload(a, device, torch.float64))
     lc, lm, li, ld = f64(log_chi), f64(log_M), f64(log_I), f64(log_D)
     if lc.dim() == 2:
         lc = lc.unsqueeze(0)
-    res_t = torch.from_numpy(buf).to(device)
+    res_t = upload(buf, device)
     env = None
     if envelopes is not None:
         env = torch.from_numpy(np.concatenate([np.asarray(e, bool).reshape(-1) for e in envelopes]).astype(
@@ -1072,6 +1146,7 @@ def viterbi(state_types, groups, G, xs, ys, log_chi, log_M, log_I, log_D, device
     _check(lib.phmm_viterbi(ctypes.byref(md), ctypes.byref(bs), _ptr(lc), _ptr(lm), _ptr(li), _ptr(ld), _ptr(ws),
                             ctypes.c_size_t(ws.numel()), _ptr(ll), _ptr(path), _ptr(plen), _ptr(status),
                             ctypes.c_void_p(s.cuda_stream)), 'phmm_viterbi')
-    ll_h, path_h, plen_h = ll.cpu().numpy(), path.cpu().numpy(), plen.cpu().numpy()
+    h = to_host({'ll': ll, 'path': path, 'plen': plen})
+    ll_h, path_h, plen_h = h['ll'], h['path'], h['plen']
     offs = np.concatenate([[0], np.cumsum(Lx.astype(np.int64) + Ly + 1)[:-1]])
     return ll_h, [path_h[o:o + n] for o, n in zip(offs, plen_h)]

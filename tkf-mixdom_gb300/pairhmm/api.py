@@ -166,13 +166,12 @@ def _run_single_tables(chi, st, groups, EM, EI, ED, x, y, tables='FBP', cell_mas
     out = _lib.estep_tables(plan, b, want_F='F' in tables, want_B='B' in tables, want_post='P' in tables)
     Lx, Ly = len(x), len(y)
     N = len(st)
-    res = {'ll': float(out['ll'][0]), 'status': int(out['status'][0]),
-           'n_trans': out['n_trans'][0].cpu().numpy(),
-           'cnt_M': out['cnt_M'][0].cpu().numpy(), 'cnt_I': out['cnt_I'][0].cpu().numpy(),
-           'cnt_D': out['cnt_D'][0].cpu().numpy()}
+    h = _lib.to_host({k: v for k, v in out.items() if v is not None})   # one wait
+    res = {'ll': float(h['ll'][0]), 'status': int(h['status'][0])}
+    res.update({k: h[k][0].copy() for k in ('n_trans', 'cnt_M', 'cnt_I', 'cnt_D')})
     for key, name, want in (('F', 'log_F', 'F'), ('B', 'log_B', 'B'), ('post', 'post', 'P')):
         if want in tables:
-            res[key] = out[name].cpu().numpy().reshape(Lx + 1, Ly + 1, N)
+            res[key] = h[name].reshape(Lx + 1, Ly + 1, N)
     return res
 
 
@@ -818,8 +817,7 @@ def estep_1d_mixdom2(params, cols, ancs, descs, ts, with_posteriors=False):
     gr = pm.mixdom_state_groups(K, F)
     lens = np.array([len(c) for c in cols], np.int64)
     off = np.concatenate([[0], np.cumsum(lens)[:-1]]).astype(np.int64)
-    cat = lambda xs: torch.from_numpy(np.concatenate([np.asarray(x, np.uint8).reshape(-1) for x in xs])
-                                      if lens.sum() else np.zeros(1, np.uint8)).to(dev)
+    cat = lambda xs: _lib.upload(_lib.concat_u8(xs) if lens.sum() else np.zeros(1, np.uint8), dev)
     emit, st1 = _lib.fb1d_emissions(st, gr, K * F, lens, off, cat(cols), cat(ancs), cat(descs), EM, EI, ED, True)
     ll, nt, post, st2 = _lib.fb1d(len(st), lens, off, emit, chi, True, 0, 1, posteriors=with_posteriors)
     res = {'log_p': ll, 'n_trans': nt, 'status': st1 | st2}
@@ -841,11 +839,15 @@ class ConstrainedLogLik(torch.autograd.Function):
         N, G = len(st), EM.shape[1]
         lens = np.array([len(c) for c in cols], np.int64)
         off = np.concatenate([[0], np.cumsum(lens)[:-1]]).astype(np.int64)
-        cat = lambda xs: (np.concatenate([np.asarray(x, np.int64).reshape(-1) for x in xs])
-                          if lens.sum() else np.zeros(1, np.int64))
-        c_all, a_all, d_all = cat(cols), cat(ancs), cat(descs)
-        to_u8 = lambda a: torch.from_numpy(np.clip(a, 0, 255).astype(np.uint8)).to(dev)
-        c_dev, a_dev, d_dev = to_u8(c_all), to_u8(a_all), to_u8(d_all)
+
+        def codes(xs):   # 0..255 on the device
+            if not lens.sum():
+                return _lib.upload(np.zeros(1, np.uint8), dev)
+            if all(type(x) is np.ndarray and x.dtype == np.uint8 for x in xs):
+                return _lib.upload(_lib.concat_u8(xs), dev)
+            v = np.concatenate([np.asarray(x, np.int64).reshape(-1) for x in xs])
+            return _lib.upload(np.clip(v, 0, 255).astype(np.uint8), dev)
+        c_dev, a_dev, d_dev = codes(cols), codes(ancs), codes(descs)
         f32 = lambda v: v.detach().to(torch.float32).contiguous()
         per_pair = EM.shape[0] == P
         emit, st1 = _lib.fb1d_emissions(st, gr, G, lens, off, c_dev, a_dev, d_dev, f32(EM), f32(EI), f32(ED), per_pair)
@@ -1268,10 +1270,13 @@ def _tkf92_batch(xs_pad, ys_pad, ts, Lx_real, Ly_real, lam, mu, ext, Q, pi):
     chi, EM, EI, ED, _ = _lib.tkf92_tables(lam, mu, ext, Q, pi, ts, device=dev)
     Lx_real = np.asarray(Lx_real).reshape(-1)
     Ly_real = np.asarray(Ly_real).reshape(-1)
-    xs = [np.asarray(xs_pad[b])[:int(Lx_real[b])] for b in range(len(Lx_real))]
-    ys = [np.asarray(ys_pad[b])[:int(Ly_real[b])] for b in range(len(Ly_real))]
+    packed = _lib.pack_padded(xs_pad, ys_pad, Lx_real, Ly_real)
+    xs = ys = None
+    if packed is None:
+        xs = [np.asarray(xs_pad[b])[:int(Lx_real[b])] for b in range(len(Lx_real))]
+        ys = [np.asarray(ys_pad[b])[:int(Ly_real[b])] for b in range(len(Ly_real))]
     plan = get_plan(np.array([S, M, I, D, E]), np.zeros(5, np.int32), 1)
-    return plan, _lib.make_batch(xs, ys, chi, EM, EI, ED, device=dev)
+    return plan, _lib.make_batch(xs, ys, chi, EM, EI, ED, device=dev, packed=packed)
 
 
 def estep_batch_tkf92_forward_only(xs_pad, ys_pad, ts, Lx_real, Ly_real, lam, mu, ext, Q, pi):

@@ -135,7 +135,8 @@ def tkf92_bdi_epilogue(n_chi, ins_rate, del_rate, t, ext, T=None):
             and mu > 0.0 and abs(1.0 - lam / mu) >= ES_LHOPITAL_THRESHOLD and 0.0 <= x < 1.0):
         from . import _lib
         n = pm._t(n_chi).contiguous()
-        tt = pm._t(t, device=n.device).reshape(-1)
+        tt = pm._t(t, device=n.device) if isinstance(t, torch.Tensor) else _lib.upload(t, n.device, F64)
+        tt = tt.reshape(-1)
         if n.dim() == 3 and tt.numel() == n.shape[0]:
             stats, res = _lib.tkf92_bdi(n, lam, mu, tt.contiguous(), x)
             keys = ('B', 'D', 'S', 'L', 'M', 'ext_count', 'notext_count')
