@@ -124,6 +124,84 @@ __device__ void load_nest_tw(const KParams &P, int p, float *nz) {
     }
 }
 
+// ---------------------------------------------------------------- edge rows between stripes
+// A stripe's last row (forward; first row backward) goes to the stripe below
+// (above) through the edge row in global memory, and the words of a record say
+// themselves whether they are there: the rows are filled with all ones before
+// the kernels start, a bit pattern no value takes (values are results of float
+// arithmetic, whose NaN is 0x7fffffff; the exponent is stored doubled, so it is
+// even).  The producing lane stores the record and the consuming lane loads the
+// next column's early in a step and looks at it a step later, so neither executes a
+// fence: publishing progress every four columns with release and acquire held
+// both warps' steps for the L2 round trips (17 states, a 127 x 1200 pair: 0.99 us a
+// step against 0.77 for a lone stripe; now 0.80).  The progress word remains for the
+// count pass (Ly + 2 when the stripe is done) and for a stripe that gave up (Ly + 1).
+__device__ __forceinline__ uint4 ld_edge4(const float *p) {
+    uint4 v;
+    asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_edge4(float *p, float a, float b, float c, float d) {
+    asm volatile("st.relaxed.gpu.global.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+__device__ __forceinline__ int ld_edge(const int *p) {
+    int v;
+    asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_edge_exp(int *p, int e) {
+    asm volatile("st.relaxed.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(2 * e) : "memory");
+}
+
+// A column of the neighbour stripe's edge row, in flight or there.
+template <int SP>
+struct EdgeColumn {
+    float v[SP];
+    int e2, col;   // doubled exponent; the column the words belong to, or -1
+    __device__ __forceinline__ void clear(int c) {   // a column the cell mask leaves empty
+#pragma unroll
+        for (int s = 0; s < SP; ++s) v[s] = 0.f;
+        e2 = 2 * EXP_NONE;
+        col = c;
+    }
+    __device__ __forceinline__ void load(const float *row, const int *rowE, int c) {
+        const float *src = row + (int64_t)c * SP;
+#pragma unroll
+        for (int q = 0; q < SP / 4; ++q) {
+            const uint4 w = ld_edge4(src + 4 * q);
+            v[4 * q] = __uint_as_float(w.x);
+            v[4 * q + 1] = __uint_as_float(w.y);
+            v[4 * q + 2] = __uint_as_float(w.z);
+            v[4 * q + 3] = __uint_as_float(w.w);
+        }
+        e2 = ld_edge(rowE + c);
+        col = c;
+    }
+    __device__ __forceinline__ bool there() const {
+        unsigned m = (unsigned)e2 == 0xffffffffu ? 0xffffffffu : 0u;
+#pragma unroll
+        for (int s = 0; s < SP; ++s) m = max(m, __float_as_uint(v[s]));
+        return m != 0xffffffffu;
+    }
+    // Until column c is there: false when the bound is hit first.  A neighbour
+    // that gave up (or ended) without it leaves zeros.
+    __device__ bool wait(const float *row, const int *rowE, int c, const int *prog, int Ly, long long limit) {
+        if (col != c) load(row, rowE, c);
+        for (long long it = 0; !there(); ++it) {
+            if (it > limit) return false;
+            const bool over = (it & 7) == 7 && ld_acquire(prog) > Ly;
+            if (it > 3) __nanosleep(64);
+            load(row, rowE, c);
+            if (over && !there()) {
+                clear(c);
+                break;
+            }
+        }
+        return true;
+    }
+};
+
 // MK: the batch carries a cell mask (a separate instantiation, so the
 // unmasked recursion carries none of the mask's instructions)
 // NT: NoNest (dense chi) or Nest<K, F> (factored MixDom transitions, unmasked batches)
@@ -218,46 +296,30 @@ __device__ void fwd_stripe_tw(const KParams &P, int p, int si, const SmemTW &LT,
     };
     load_emit(t_beg);
     bool aborted = false;
-    float hx[SP];
-#pragma unroll
-    for (int s = 0; s < SP; ++s) hx[s] = 0.f;
-    int hxE = EXP_NONE, hx_col = -1, pv = 0;
-    if (si > 0 && r == 0) pv = ld_acquire(prog_above);
+    EdgeColumn<SP> hx;
+    hx.clear(-1);
     // a stripe that starts past step 0: row 0's first M predecessor is column
     // t_beg - 1 of the row above, which the skipped step t_beg - 1 would have
     // read -- load it into the history here
     if (MK && si > 0 && r == 0 && t_beg <= t_end && t_beg - 1 >= max(hlo, 0) && t_beg - 1 <= hhi) {
-        const int col = t_beg - 1;
-        if (!wait_geq(prog_above, col + 1, P.spin_limit)) {
+        if (!hx.wait(edge_above, edgeE_above, t_beg - 1, prog_above, Ly, P.spin_limit)) {
             s_abort[t_beg & 1] = 1;   // seen by all threads after the first step's barrier
         } else {
-            const float *src = edge_above + (int64_t)col * SP;
 #pragma unroll
-            for (int q = 0; q < SQ; ++q) m0[q] = make_float2(__ldcg(src + 2 * q), __ldcg(src + 2 * q + 1));
-            Em0 = __ldcg(edgeE_above + col);
+            for (int q = 0; q < SQ; ++q) m0[q] = make_float2(hx.v[2 * q], hx.v[2 * q + 1]);
+            Em0 = hx.e2 >> 1;
         }
     }
 
     for (int t = t_beg; t <= t_end; ++t) {
-        // halo (row i0-1, column t) for thread 0: normally prefetched during
-        // step t-1; zero off the live columns above (a cell mask)
-        if (si > 0 && t <= Ly && r == 0 && hx_col != t) {
+        // halo (row i0-1, column t) for thread 0, loaded during step t-1; zero
+        // off the live columns above (a cell mask)
+        if (si > 0 && t <= Ly && r == 0) {
             if (MK && (t < hlo || t > hhi)) {
-#pragma unroll
-                for (int s = 0; s < SP; ++s) hx[s] = 0.f;
-                hxE = EXP_NONE;
-                hx_col = t;
-            } else if (!wait_geq(prog_above, t + 1, P.spin_limit)) {
+                hx.clear(t);
+            } else if (!hx.wait(edge_above, edgeE_above, t, prog_above, Ly, P.spin_limit)) {
                 s_abort[t & 1] = 1;   // read by all threads after this step's barrier
-            } else {
-                const float4 *src = reinterpret_cast<const float4 *>(edge_above + (int64_t)t * SP);
-#pragma unroll
-                for (int q = 0; q < SP / 4; ++q) {
-                    const float4 v = __ldcg(src + q);
-                    hx[4 * q] = v.x; hx[4 * q + 1] = v.y; hx[4 * q + 2] = v.z; hx[4 * q + 3] = v.w;
-                }
-                hxE = __ldcg(edgeE_above + t);
-                hx_col = t;
+                hx.clear(t);
             }
         }
         const int jc = t - r;
@@ -279,15 +341,18 @@ __device__ void fwd_stripe_tw(const KParams &P, int p, int si, const SmemTW &LT,
         }
         const bool l0 = lane == 0, top = r == 0;
         int EdA = __shfl_up_sync(0xffffffffu, Eprev, 1);
-        EdA = l0 ? (top ? (halo ? hxE : EXP_NONE) : bndE[slot]) : EdA;
+        EdA = l0 ? (top ? (halo ? hx.e2 >> 1 : EXP_NONE) : bndE[slot]) : EdA;
 #pragma unroll
         for (int q = 0; q < SQ; ++q) {
             if (2 * q >= NSRC) continue;   // padding pairs stay zero
             const float vx = __shfl_up_sync(0xffffffffu, prev[q].x, 1);
             const float vy = __shfl_up_sync(0xffffffffu, prev[q].y, 1);
-            d0[q].x = l0 ? (top ? (halo ? hx[2 * q] : 0.f) : bv[2 * q]) : vx;
-            d0[q].y = l0 ? (top ? (halo ? hx[2 * q + 1] : 0.f) : bv[2 * q + 1]) : vy;
+            d0[q].x = l0 ? (top ? (halo ? hx.v[2 * q] : 0.f) : bv[2 * q]) : vx;
+            d0[q].y = l0 ? (top ? (halo ? hx.v[2 * q + 1] : 0.f) : bv[2 * q + 1]) : vy;
         }
+        // the next halo column, a whole step ahead of its use
+        if (si > 0 && r == 0 && t + 1 <= Ly && !(MK && (t + 1 < hlo || t + 1 > hhi)))
+            hx.load(edge_above, edgeE_above, t + 1);
         // a type that may not emit here contributes nothing (nor its exponent);
         // outside the lattice nothing emits, so the type scales below are zero
         // there and no separate select clears the cell
@@ -432,7 +497,7 @@ __device__ void fwd_stripe_tw(const KParams &P, int p, int si, const SmemTW &LT,
                 P.lat_exp[latc + (int64_t)t * ROWS + r] = Enew;
             }
             if (has_below && r == ROWS - 1) {
-                float4 *dst = reinterpret_cast<float4 *>(edge_mine + (int64_t)jc * SP);
+                float *dst = edge_mine + (int64_t)jc * SP;
 #pragma unroll
                 for (int q = 0; q < SP / 4; ++q) {
                     float v[4];
@@ -441,10 +506,9 @@ __device__ void fwd_stripe_tw(const KParams &P, int p, int si, const SmemTW &LT,
                         const int s = 4 * q + u;
                         v[u] = s < NE ? acc[s] : (s == NE ? sNew : 0.f);
                     }
-                    dst[q] = make_float4(v[0], v[1], v[2], v[3]);
+                    st_edge4(dst + 4 * q, v[0], v[1], v[2], v[3]);
                 }
-                edgeE_mine[jc] = Enew;
-                if (((jc + 1) % PUB) == 0 || jc == t_end - (ROWS - 1)) st_release(prog_mine, jc + 1);
+                st_edge_exp(edgeE_mine + jc, Enew);
             }
             if (rowi == Lx && jc == Ly && si + 1 == m.n_stripes) {
                 double a = 0.0;
@@ -484,26 +548,6 @@ __device__ void fwd_stripe_tw(const KParams &P, int p, int si, const SmemTW &LT,
             bndE[t & 1] = Eprev;
         }
         load_emit(t + 1);
-        // prefetch halo column t+1 when the progress read last step covers it
-        // (its loads then overlap the barrier), and poll for the column after
-        if (si > 0 && r == 0 && t + 1 <= Ly) {
-            if (MK && (t + 1 < hlo || t + 1 > hhi)) {
-#pragma unroll
-                for (int s = 0; s < SP; ++s) hx[s] = 0.f;
-                hxE = EXP_NONE;
-                hx_col = t + 1;
-            } else if (pv > t + 1) {
-                const float4 *src = reinterpret_cast<const float4 *>(edge_above + (int64_t)(t + 1) * SP);
-#pragma unroll
-                for (int q = 0; q < SP / 4; ++q) {
-                    const float4 v = __ldcg(src + q);
-                    hx[4 * q] = v.x; hx[4 * q + 1] = v.y; hx[4 * q + 2] = v.z; hx[4 * q + 3] = v.w;
-                }
-                hxE = __ldcg(edgeE_above + t + 1);
-                hx_col = t + 1;
-            }
-            if (t + 2 <= hhi && pv <= t + 2) pv = ld_acquire(prog_above);
-        }
         __syncthreads();
         // the flag of step t is written only before this barrier, and the
         // next write goes to the other parity: every thread sees the same value
@@ -616,52 +660,37 @@ __device__ void bwd_rec_stripe_tw(const KParams &P, int p, int si, const SmemTW 
     };
     load_emit(t_end);
     bool aborted = false;
-    float hx[SP];
-#pragma unroll
-    for (int s = 0; s < SP; ++s) hx[s] = 0.f;
-    int hxE = EXP_NONE, hx_col = -1, pv = 0;
-    if (has_below && r == ROWS - 1) pv = ld_acquire(prog_below);
+    EdgeColumn<SP> hx;
+    hx.clear(-1);
     // a stripe that ends before its last step: row 63's first M successor is
     // column jb + 1 of the row below (jb = t_end - 63), which the skipped step
     // t_end + 1 would have received -- load it into the history here
     if (MK && has_below && r == ROWS - 1 && t_beg <= t_end) {
         const int col = t_end - (ROWS - 1) + 1;
         if (col >= max(hlo, 0) && col <= hhi) {
-            if (!wait_geq(prog_below, Ly + 1 - col, P.spin_limit)) {
+            if (!hx.wait(edge_below, edgeE_below, col, prog_below, Ly, P.spin_limit)) {
                 s_abort[t_end & 1] = 1;   // seen by all threads after the first step's barrier
             } else {
-                const float *src = edge_below + (int64_t)col * SP;
 #pragma unroll
                 for (int q = 0; q < KQ; ++q) {
                     if (2 * q >= NE) continue;
-                    mR[q] = make_float2(__ldcg(src + 2 * q), __ldcg(src + 2 * q + 1));
+                    mR[q] = make_float2(hx.v[2 * q], hx.v[2 * q + 1]);
                 }
-                EmR = __ldcg(edgeE_below + col);
+                EmR = hx.e2 >> 1;
             }
         }
     }
 
     for (int t = t_end; t >= t_beg; --t) {
         const int jb = t - (ROWS - 1);
-        // halo (row i0+64, column jb) for thread 63: normally prefetched during
-        // step t+1; zero off the live columns below (a cell mask)
-        if (has_below && jb >= 0 && jb <= Ly && r == ROWS - 1 && hx_col != jb) {
+        // halo (row i0+64, column jb) for thread 63, loaded during step t+1; zero
+        // off the live columns below (a cell mask)
+        if (has_below && jb >= 0 && jb <= Ly && r == ROWS - 1) {
             if (MK && (jb < hlo || jb > hhi)) {
-#pragma unroll
-                for (int s = 0; s < SP; ++s) hx[s] = 0.f;
-                hxE = EXP_NONE;
-                hx_col = jb;
-            } else if (!wait_geq(prog_below, Ly + 1 - jb, P.spin_limit)) {
+                hx.clear(jb);
+            } else if (!hx.wait(edge_below, edgeE_below, jb, prog_below, Ly, P.spin_limit)) {
                 s_abort[t & 1] = 1;   // read by all threads after this step's barrier
-            } else {
-                const float4 *src = reinterpret_cast<const float4 *>(edge_below + (int64_t)jb * SP);
-#pragma unroll
-                for (int q = 0; q < SP / 4; ++q) {
-                    const float4 v = __ldcg(src + q);
-                    hx[4 * q] = v.x; hx[4 * q + 1] = v.y; hx[4 * q + 2] = v.z; hx[4 * q + 3] = v.w;
-                }
-                hxE = __ldcg(edgeE_below + jb);
-                hx_col = jb;
+                hx.clear(jb);
             }
         }
         const int jc = t - r;
@@ -681,15 +710,18 @@ __device__ void bwd_rec_stripe_tw(const KParams &P, int p, int si, const SmemTW 
         }
         const bool l31 = lane == 31, bottom = r == ROWS - 1;
         int EdRn = __shfl_down_sync(0xffffffffu, Ewn, 1);
-        EdRn = l31 ? (bottom ? (halo ? hxE : EXP_NONE) : bndE[slot]) : EdRn;
+        EdRn = l31 ? (bottom ? (halo ? hx.e2 >> 1 : EXP_NONE) : bndE[slot]) : EdRn;
 #pragma unroll
         for (int q = 0; q < KQ; ++q) {
             if (2 * q >= NE) continue;   // padding pairs stay zero
             const float vx = __shfl_down_sync(0xffffffffu, wn[q].x, 1);
             const float vy = __shfl_down_sync(0xffffffffu, wn[q].y, 1);
-            dR[q].x = l31 ? (bottom ? (halo ? hx[2 * q] : 0.f) : bv[2 * q]) : vx;
-            dR[q].y = l31 ? (bottom ? (halo ? hx[2 * q + 1] : 0.f) : bv[2 * q + 1]) : vy;
+            dR[q].x = l31 ? (bottom ? (halo ? hx.v[2 * q] : 0.f) : bv[2 * q]) : vx;
+            dR[q].y = l31 ? (bottom ? (halo ? hx.v[2 * q + 1] : 0.f) : bv[2 * q + 1]) : vy;
         }
+        // the next halo column, a whole step ahead of its use
+        if (has_below && r == ROWS - 1 && jb - 1 >= 0 && jb - 1 <= Ly && !(MK && (jb - 1 < hlo || jb - 1 > hhi)))
+            hx.load(edge_below, edgeE_below, jb - 1);
         const bool term = valid && rowi == Lx && jc == Ly;
         const bool hI = jc + 1 <= Ly, hD = rowi + 1 <= Lx, hM = hI && hD;
         const int EI = hI ? Ewn : EXP_NONE, ED = hD ? EdRn : EXP_NONE, EM = hM ? EmR : EXP_NONE;
@@ -839,7 +871,7 @@ __device__ void bwd_rec_stripe_tw(const KParams &P, int p, int si, const SmemTW 
             }
             P.blat_exp[latc + (int64_t)t * ROWS + r] = Eb;
             if (has_above && rowi == i0) {   // top row -> edge for the stripe above
-                float4 *e = reinterpret_cast<float4 *>(edge_mine + (int64_t)jc * SP);
+                float *e = edge_mine + (int64_t)jc * SP;
 #pragma unroll
                 for (int q = 0; q < SP / 4; ++q) {
                     float v[4];
@@ -848,10 +880,9 @@ __device__ void bwd_rec_stripe_tw(const KParams &P, int p, int si, const SmemTW 
                         const int k = 4 * q + u;
                         v[u] = k < NE ? wnew[k] : 0.f;
                     }
-                    e[q] = make_float4(v[0], v[1], v[2], v[3]);
+                    st_edge4(e + 4 * q, v[0], v[1], v[2], v[3]);
                 }
-                edgeE_mine[jc] = Eb;
-                if ((jc % PUB) == 0 || jc == t_beg) st_release(prog_mine, Ly + 1 - jc);
+                st_edge_exp(edgeE_mine + jc, Eb);
             }
         }
 #pragma unroll
@@ -873,26 +904,6 @@ __device__ void bwd_rec_stripe_tw(const KParams &P, int p, int si, const SmemTW 
             bndE[t & 1] = Ewn;
         }
         load_emit(t - 1);
-        // prefetch halo column jb-1 when the progress read last step covers it,
-        // and poll for the column after
-        if (has_below && r == ROWS - 1 && jb - 1 >= 0 && jb - 1 <= Ly) {
-            if (MK && (jb - 1 < hlo || jb - 1 > hhi)) {
-#pragma unroll
-                for (int s = 0; s < SP; ++s) hx[s] = 0.f;
-                hxE = EXP_NONE;
-                hx_col = jb - 1;
-            } else if (pv >= Ly + 1 - (jb - 1)) {
-                const float4 *src = reinterpret_cast<const float4 *>(edge_below + (int64_t)(jb - 1) * SP);
-#pragma unroll
-                for (int q = 0; q < SP / 4; ++q) {
-                    const float4 v = __ldcg(src + q);
-                    hx[4 * q] = v.x; hx[4 * q + 1] = v.y; hx[4 * q + 2] = v.z; hx[4 * q + 3] = v.w;
-                }
-                hxE = __ldcg(edgeE_below + jb - 1);
-                hx_col = jb - 1;
-            }
-            if (jb - 2 >= hlo && pv < Ly + 3 - jb) pv = ld_acquire(prog_below);
-        }
         __syncthreads();
         // the flag of step t is written only before this barrier, and the
         // next write goes to the other parity: every thread sees the same value

@@ -1086,12 +1086,10 @@ struct phmm_plan {
     float *lat = nullptr; size_t lat_cap = 0;
     int *lat_exp = nullptr; size_t latE_cap = 0;
     float *edge = nullptr; size_t edge_cap = 0;
-    int *edge_exp = nullptr; size_t edgeE_cap = 0;
     int *progress = nullptr; size_t prog_cap = 0;
     float *blat = nullptr; size_t blat_cap = 0;      // split E-step
     int *blat_exp = nullptr; size_t blatE_cap = 0;
     float *bedge = nullptr; size_t bedge_cap = 0;
-    int *bedge_exp = nullptr; size_t bedgeE_cap = 0;
     int64_t *slat = nullptr; size_t slat_cap = 0;    // checkpointed wide E-step: stripe offsets per group
     // split E-step: one side stream (+ fork / join events) per caller stream
     // (prio: the wavefront streams were created at the greatest priority and the
@@ -1941,14 +1939,15 @@ int run_core(phmm_plan *plan, const phmm_batch *b, bool estep, double *ll, doubl
     const size_t o_cnt = align256(o_items + sizeof(int2) * (plan->h_items.size() + n_range));
     const size_t o_prog = align256(o_cnt + 4 * sizeof(int));
     const size_t o_edge = align256(o_prog + sizeof(int) * 2 * (size_t)stripes);
-    const size_t o_edgeE = align256(o_edge + sizeof(float) * (size_t)edge_cells * stride);
-    const size_t o_lat = align256(o_edgeE + sizeof(int) * (size_t)edge_cells * estride);
+    // the edge rows of both directions and their exponents lie in one piece (one fill)
+    const size_t n_edge = align256(sizeof(float) * (size_t)edge_cells * stride);
+    const size_t n_edgeE = align256(sizeof(int) * (size_t)edge_cells * estride);
+    const size_t edge_bytes = (split ? 2 : 1) * (n_edge + n_edgeE);
+    const size_t o_lat = o_edge + edge_bytes;
     const size_t o_latE = align256(o_lat + (estep ? sizeof(float) * (size_t)lat_cells * stride : 0));
     const size_t o_blat = align256(o_latE + (estep ? sizeof(int) * (size_t)lat_cells * estride : 0));
     const size_t o_blatE = align256(o_blat + (split ? sizeof(float) * (size_t)lat_cells * stride : 0));
-    const size_t o_bedge = align256(o_blatE + (split ? sizeof(int) * (size_t)lat_cells * estride : 0));
-    const size_t o_bedgeE = align256(o_bedge + (split ? sizeof(float) * (size_t)edge_cells * stride : 0));
-    const size_t need = align256(o_bedgeE + (split ? sizeof(int) * (size_t)edge_cells * estride : 0));
+    const size_t need = align256(o_blatE + (split ? sizeof(int) * (size_t)lat_cells * estride : 0));
     if (ws_need) { *ws_need = need; return 0; }
     void *d_meta, *d_items;
     int *d_counters, *d_progress, *d_edge_exp, *d_lat_exp, *d_blat_exp = nullptr, *d_bedge_exp = nullptr;
@@ -1966,21 +1965,17 @@ int run_core(phmm_plan *plan, const phmm_batch *b, bool estep, double *ll, doubl
         d_counters = (int *)(w + o_cnt);
         d_progress = (int *)(w + o_prog);
         d_edge = (float *)(w + o_edge);
-        d_edge_exp = (int *)(w + o_edgeE);
         d_lat = estep ? (float *)(w + o_lat) : nullptr;
         d_lat_exp = estep ? (int *)(w + o_latE) : nullptr;
         if (split) {
             d_blat = (float *)(w + o_blat);
             d_blat_exp = (int *)(w + o_blatE);
-            d_bedge = (float *)(w + o_bedge);
-            d_bedge_exp = (int *)(w + o_bedgeE);
         }
     } else {
         if ((rc = ensure((char **)&plan->meta, &plan->meta_cap, sizeof(PairMeta) * P_))) return rc;
         if ((rc = ensure((char **)&plan->items, &plan->items_cap, sizeof(int2) * (plan->h_items.size() + n_range))))
             return rc;
-        if ((rc = ensure(&plan->edge, &plan->edge_cap, (size_t)edge_cells * stride))) return rc;
-        if ((rc = ensure(&plan->edge_exp, &plan->edgeE_cap, (size_t)edge_cells * estride))) return rc;
+        if ((rc = ensure(&plan->edge, &plan->edge_cap, edge_bytes / sizeof(float)))) return rc;
         if ((rc = ensure(&plan->progress, &plan->prog_cap, (size_t)2 * stripes))) return rc;
         if (estep) {
             if ((rc = ensure(&plan->lat, &plan->lat_cap, (size_t)lat_cells * stride))) return rc;
@@ -1991,19 +1986,19 @@ int run_core(phmm_plan *plan, const phmm_batch *b, bool estep, double *ll, doubl
         d_counters = plan->counters;
         d_progress = plan->progress;
         d_edge = plan->edge;
-        d_edge_exp = plan->edge_exp;
         d_lat = plan->lat;
         d_lat_exp = plan->lat_exp;
         if (split) {
             if ((rc = ensure(&plan->blat, &plan->blat_cap, (size_t)lat_cells * stride))) return rc;
             if ((rc = ensure(&plan->blat_exp, &plan->blatE_cap, (size_t)lat_cells * estride))) return rc;
-            if ((rc = ensure(&plan->bedge, &plan->bedge_cap, (size_t)edge_cells * stride))) return rc;
-            if ((rc = ensure(&plan->bedge_exp, &plan->bedgeE_cap, (size_t)edge_cells * estride))) return rc;
             d_blat = plan->blat;
             d_blat_exp = plan->blat_exp;
-            d_bedge = plan->bedge;
-            d_bedge_exp = plan->bedge_exp;
         }
+    }
+    d_edge_exp = (int *)((unsigned char *)d_edge + n_edge);
+    if (split) {
+        d_bedge = (float *)((unsigned char *)d_edge_exp + n_edgeE);
+        d_bedge_exp = (int *)((unsigned char *)d_bedge + n_edge);
     }
     if (plan->desc_mode != 2) {   // the work description (launch-only calls find it in the workspace)
         CUDA_TRY(cudaMemcpyAsync(d_meta, plan->h_meta.data(), sizeof(PairMeta) * P_, cudaMemcpyHostToDevice,
@@ -2069,6 +2064,8 @@ int run_core(phmm_plan *plan, const phmm_batch *b, bool estep, double *ll, doubl
         plan->launches++;
         K.srange = range;
     }
+    if (two_warp && stripes > P_)   // no word of an edge row is there yet (EdgeColumn)
+        CUDA_TRY(cudaMemsetAsync(d_edge, 0xff, edge_bytes, stream));
     if (split) return launch_split(plan, K, wl ? wl : bl, bl != nullptr, n_items, n_citems, stripes, max_ly, d_items,
                                    d_counters, d_progress, d_bedge, d_bedge_exp, stream);
     for (int pass = 0; pass < (estep ? 2 : 1); ++pass) {
@@ -2226,8 +2223,7 @@ int launch_warp(phmm_plan *plan, KParams &K, int n_items, int max_ly, int kind, 
 size_t plan_scratch_bytes(const phmm_plan *plan) {
     return plan->meta_cap + plan->items_cap + sizeof(int64_t) * plan->slat_cap +
            sizeof(float) * (plan->lat_cap + plan->edge_cap + plan->blat_cap +
-           plan->bedge_cap) + sizeof(int) * (plan->latE_cap + plan->edgeE_cap + plan->prog_cap + plan->blatE_cap +
-           plan->bedgeE_cap);
+           plan->bedge_cap) + sizeof(int) * (plan->latE_cap + plan->prog_cap + plan->blatE_cap);
 }
 
 int run_groups(phmm_plan *plan, const phmm_batch *b, bool estep, double *ll, double *n_trans, double *cntM,
@@ -2475,14 +2471,12 @@ void phmm_plan_destroy(phmm_plan *plan) {
     cudaFree(plan->blat);
     cudaFree(plan->blat_exp);
     cudaFree(plan->bedge);
-    cudaFree(plan->bedge_exp);
     cudaFree(plan->meta);
     cudaFree(plan->items);
     cudaFree(plan->counters);
     cudaFree(plan->lat);
     cudaFree(plan->lat_exp);
     cudaFree(plan->edge);
-    cudaFree(plan->edge_exp);
     cudaFree(plan->progress);
     cudaFree(plan->slat);
     delete plan;
