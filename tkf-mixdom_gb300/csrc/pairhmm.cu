@@ -250,6 +250,19 @@ __device__ int count_claim(const KParams &P) {
     return atomicAdd(P.counter, 1);
 }
 
+// Ahead of the overlapped count grid on its stream: holds one thread, not half the
+// GPU's slots, until both wavefront kernels have claimed a stripe (or the window
+// has passed, as in count_claim).  Count CTAs that became resident between the two
+// kernels kept the second from starting until their window ended: 64 banded
+// TKF92 pairs took 1.55 ms or 1.75 ms by which came first.
+__global__ void count_gate_kernel(const int *wave_ctr) {
+    const unsigned long long t0 = globaltimer_ns();
+    while (ld_acquire(wave_ctr) == 0 || ld_acquire(wave_ctr + 1) == 0) {
+        if (globaltimer_ns() - t0 > COUNT_START_WINDOW_NS) return;
+        __nanosleep(256);
+    }
+}
+
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
     unsigned s = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
@@ -993,53 +1006,119 @@ __global__ void __launch_bounds__(512) backward_kernel(const KParams P) {
 // the recursions skip those anti-diagonal steps.
 constexpr int RANGE_EMPTY_LO = 1 << 30, RANGE_EMPTY_HI = -(1 << 30);
 
-__global__ void stripe_range_kernel(const KParams P, int rows, int2 *range) {
+// Warps take rows; a row is read as the 16-byte words inside it and the bytes at
+// its ends (a byte at a time, rows one after the other: 66 us for 64 pairs of 500
+// x 500, two dependent loads a row; now 16 us).
+__global__ void __launch_bounds__(256) stripe_range_kernel(const KParams P, int rows, int2 *range) {
     const int2 w = P.items[blockIdx.x];
     const PairMeta m = P.meta[w.x];
     const int si = w.y, i0 = si * rows, nrows = min(rows, m.Lx + 1 - i0);
+    const int lane = threadIdx.x & 31, n = m.Ly + 1;
     __shared__ int s_lo, s_hi;
     if (threadIdx.x == 0) { s_lo = RANGE_EMPTY_LO; s_hi = RANGE_EMPTY_HI; }
     __syncthreads();
     int lo = RANGE_EMPTY_LO, hi = RANGE_EMPTY_HI;
-    for (int r = 0; r < nrows; ++r) {
-        const unsigned char *row = P.cmask + m.tab_base + (int64_t)(i0 + r) * (m.Ly + 1);
-        for (int j = threadIdx.x; j <= m.Ly; j += blockDim.x)
+    auto word = [&](unsigned v, int j) {   // bytes j..j+3 of a row
+        if (!v) return;
+        lo = min(lo, j + ((__ffs(v) - 1) >> 3));
+        hi = max(hi, j + ((31 - __clz(v)) >> 3));
+    };
+#pragma unroll 4
+    for (int r = threadIdx.x >> 5; r < nrows; r += 8) {
+        const unsigned char *row = P.cmask + m.tab_base + (int64_t)(i0 + r) * n;
+        const int head = min(n, (int)(-(intptr_t)row & 15)), nv = (n - head) >> 4, tail = head + 16 * nv;
+        const int j = lane < 16 ? lane : tail + lane - 16;   // head < 16, n - tail < 16
+        if (lane < 16 ? j < head : j < n)
             if (row[j]) { lo = min(lo, j); hi = max(hi, j); }
+        for (int q = lane; q < nv; q += 32) {
+            const uint4 v = __ldg(reinterpret_cast<const uint4 *>(row + head) + q);
+            const int j0 = head + 16 * q;
+            word(v.x, j0);
+            word(v.y, j0 + 4);
+            word(v.z, j0 + 8);
+            word(v.w, j0 + 12);
+        }
     }
     if (si + 1 == m.n_stripes && threadIdx.x == 0) { lo = min(lo, m.Ly); hi = max(hi, m.Ly); }
-    if (lo <= hi) { atomicMin(&s_lo, lo); atomicMax(&s_hi, hi); }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if (lane == 0 && lo <= hi) { atomicMin(&s_lo, lo); atomicMax(&s_hi, hi); }
     __syncthreads();
     if (threadIdx.x == 0) range[m.stripe_base + si] = make_int2(s_lo, s_hi);
+}
+
+// f b 2^e as a double: the significands' product is exact in 48 bits, so the
+// integer units build the number (two conversions and two products on the FP64
+// unit are four of its issues a value)
+__device__ __forceinline__ double product_pow2(float f, float b, int e) {
+    const unsigned uf = __float_as_uint(f), ub = __float_as_uint(b);
+    const int ef = (int)((uf >> 23) & 255), eb = (int)((ub >> 23) & 255);
+    if (f == 0.f || b == 0.f) return 0.0;
+    const int ex = ef + eb - 254 + e + 1023;
+    if (ef == 0 || ef == 255 || eb == 0 || eb == 255 || ex < 1 || ex > 2045)   // subnormal, not finite or far out
+        return scalbn((double)f * (double)b, e);
+    const uint64_t prod = (uint64_t)((uf & 0x7fffffu) | 0x800000u) * ((ub & 0x7fffffu) | 0x800000u);
+    const int top = (int)(prod >> 47);   // leading bit at 47 or at 46
+    const uint64_t frac = (prod << (6 - top)) & 0xfffffffffffffull;
+    return __longlong_as_double((long long)(((uint64_t)((uf ^ ub) >> 31) << 63) | ((uint64_t)(ex + top) << 52) | frac));
 }
 
 // Band-layout posteriors from the split E-step's two-warp lattices: one CTA
 // per forward stripe item; position (i, b) of a pair's rows takes
 // f~ b~ 2^(Ef + Eb) / P at cell (i, center[i] - W + b) for the emitting
-// states and the start (source slots 0..nsrc-1, start last); cells off the
-// stripe's live columns or off the lattice stay 0 (set by the caller).
-__global__ void band_post_kernel(const KParams P, int rows, int stride, int nsrc, const int32_t *center, int W,
-                                 double *out) {
+// states and the start (source slots 0..nsrc-1, start last), and zero off the
+// stripe's live columns, off the lattice and for the other states.
+//
+// A stripe's rows are one piece of the output, so a warp takes 32 positions of it, stages
+// their states in shared memory and writes them in order.  1/P is one power of two and one factor
+// in [1/2, 1) a CTA (an exp2 a cell and FP64 conversions a value: 191 us at 64
+// pairs of 500 rows by 73 columns, 5 states; now 78 us, 93 MB written).
+constexpr int BAND_THREADS = 256;
+
+__global__ void __launch_bounds__(BAND_THREADS) band_post_kernel(const KParams P, int rows, int stride, int nsrc,
+                                                                 const int32_t *center, int W, double *out) {
+    extern __shared__ double band_stage[];
     const int2 w = P.items[blockIdx.x];
-    const int p = w.x, si = w.y;
+    const int p = w.x, si = w.y, N = P.N;
     const PairMeta m = P.meta[p];
     const double llv = P.ll[p];
-    if (!(llv > -1e29)) return;
-    const double lam = llv / LN2;
+    const bool live = llv > -1e29;
+    const double lam = llv / LN2, whole = floor(lam);
+    const double c = live ? exp2(whole - lam) : 0.0;
+    const int Ep = live ? (int)whole : 0;
     const int i0 = si * rows, nrows = min(rows, m.Lx + 1 - i0), BW = 2 * W + 1;
     const int2 rg = P.srange[m.stripe_base + si];
     const int jlo = max(0, rg.x), jhi = min(m.Ly, rg.y);
     const int64_t latc = m.lat_base + (int64_t)si * (rows + m.Ly) * rows;
-    for (int idx = threadIdx.x; idx < nrows * BW; idx += blockDim.x) {
-        const int r = idx / BW, b = idx - r * BW, i = i0 + r;
-        const int j = center[m.row_base + i] - W + b;
-        if (j < jlo || j > jhi) continue;
-        const int64_t cell = latc + (int64_t)(j + r) * rows + r;
-        const int Ef = P.lat_exp[cell], Eb = P.blat_exp[cell];
-        if (Ef <= EXP_NONE || Eb <= EXP_NONE) continue;
-        const double sc = exp2((double)(Ef + Eb) - lam);
-        double *o = out + ((m.row_base + i) * BW + b) * P.N;
-        for (int s = 0; s < nsrc; ++s)
-            o[P.w_orig[s]] = (double)P.lat[cell * stride + s] * (double)P.blat[cell * stride + s] * sc;
+    const int lane = threadIdx.x & 31, n = nrows * BW;
+    double *stage = band_stage + (threadIdx.x >> 5) * 32 * N, *mine = stage + lane * N;
+    double *o = out + (m.row_base + i0) * BW * N;
+    for (int base = threadIdx.x & ~31; base < n; base += BAND_THREADS) {
+        const int idx = base + lane;
+        for (int s = 0; s < N; ++s) mine[s] = 0.0;
+        if (live && idx < n) {
+            const int r = idx / BW, b = idx - r * BW;
+            const int j = center[m.row_base + i0 + r] - W + b;
+            if (j >= jlo && j <= jhi) {
+                const int64_t cell = latc + (int64_t)(j + r) * rows + r;
+                const int Ef = P.lat_exp[cell], Eb = P.blat_exp[cell];
+                if (Ef > EXP_NONE && Eb > EXP_NONE) {
+                    const float4 *fr = reinterpret_cast<const float4 *>(P.lat + cell * stride);
+                    const float4 *br = reinterpret_cast<const float4 *>(P.blat + cell * stride);
+                    for (int s = 0; s < nsrc; s += 4) {
+                        const float4 f = fr[s / 4], g = br[s / 4];
+                        const float fv[4] = {f.x, f.y, f.z, f.w}, gv[4] = {g.x, g.y, g.z, g.w};
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            if (s + u < nsrc) mine[P.w_orig[s + u]] = product_pow2(fv[u], gv[u], Ef + Eb - Ep) * c;
+                    }
+                }
+            }
+        }
+        __syncwarp();
+        const int words = min(32, n - base) * N;
+        for (int k = lane; k < words; k += 32) o[(int64_t)base * N + k] = stage[k];
+        __syncwarp();
     }
 }
 
@@ -1367,6 +1446,9 @@ int launch_split(phmm_plan *plan, KParams K, WarpLauncher wl, bool combined, int
     if (tu.count_per_sm != 0) {
         plan->grid_div = 2;
         plan->launch_per_sm = tu.count_per_sm > 0 ? tu.count_per_sm : 0;
+        count_gate_kernel<<<1, 1, 0, sd->side2>>>(d_counters);
+        if (cudaError_t e = cudaGetLastError(); e != cudaSuccess) { reset(); return fail(PHMM_E_CUDA, cudaGetErrorString(e)); }
+        ++launched;
         if (plan->timing) CUDA_TRY(cudaEventRecord(plan->ev[4], sd->side2));
         rc = wl(plan, C, n_citems, max_ly, 3, sd->side2);
         reset();
@@ -2517,10 +2599,6 @@ int phmm_estep_band(phmm_plan *plan, const phmm_batch *batch, const int32_t *ban
     if (!plan->two_warp || plan->last_variant != 7)
         return fail(PHMM_E_ARG, "phmm_estep_band: the E-step did not run on the two-warp kernels");
     cudaStream_t st = (cudaStream_t)stream;
-    const int N = plan->base.N, BW = 2 * band_half_width + 1;
-    int64_t rows = 0;
-    for (int p = 0; p < batch->n_pairs; ++p) rows += batch->Lx_host[p] + 1;
-    CUDA_TRY(cudaMemsetAsync(post_band, 0, sizeof(double) * (size_t)rows * BW * N, st));
     // the E-step's work description and lattices stay in the plan's buffers;
     // the forward stripe items come first in the item list, the stripe
     // ranges right after the whole list
@@ -2537,7 +2615,8 @@ int phmm_estep_band(phmm_plan *plan, const phmm_batch *batch, const int32_t *ban
     for (int p = 0; p < batch->n_pairs; ++p) n_items += plan->h_meta[p].n_stripes;
     const int nsrc = plan->w_nm + plan->w_ni + plan->w_nd + 1;
     const int stride = (nsrc + 3) & ~3;
-    band_post_kernel<<<n_items, 256, 0, st>>>(K, warp2::ROWS, stride, nsrc, band_center, band_half_width, post_band);
+    band_post_kernel<<<n_items, BAND_THREADS, sizeof(double) * BAND_THREADS * K.N, st>>>(
+        K, warp2::ROWS, stride, nsrc, band_center, band_half_width, post_band);
     CUDA_TRY(cudaGetLastError());
     plan->launches++;
     return 0;
