@@ -1381,3 +1381,422 @@ __global__ void __launch_bounds__(TWT) count_tw_kernel(const KParams P) {
 }
 
 }  // namespace warp2
+
+// ---------------------------------------------------------------- count pass of few chunks
+// Expected counts of a chunk of CCH anti-diagonal steps of one stripe, from the
+// forward and backward lattices.  Nothing is carried from step to step but the
+// sums, so a CTA is T teams of 64 threads (one row each) that take T steps at a
+// time, and every cell reads what it needs -- its f~ and b~ and the b~ of its
+// three successors -- straight from the lattices, a round ahead.
+// A round:
+//   cells     thread (team, row): f~ scaled and u~ = w~_succ 2^(E_succ - Eb)
+//             into shared memory; M posteriors to the counts, I and D
+//             posteriors staged
+//   products  thread (team, row group, 4 x 4 tile of (source, destination)):
+//             the outer products of its rows, on packed pairs of floats
+//   sums      the compensated sums over the steps, in their order: a thread
+//             adds the T steps' partial products (or staged I and D posteriors) of its own
+//             few sums
+// The order of every float sum is that of count_chunk_tw.
+//
+// For batches with no more chunks than SMs, where a chunk's time is the pass's: one
+// pair of 60 residues at 17 states, two chunks, 116 us with count_chunk_tw's 1.75 us a
+// step, now about 85 (the call 410 -> 378 us).  It issues no fewer instructions, so with the SMs full it loses
+// (200 pairs 2.49 ms against 3.04 ms).
+namespace warp2 {
+
+constexpr int CRING = 128;   // columns of I posteriors in flight (64 + T - 1 at once)
+
+struct SmemTeams {
+    int tM, tI, tD, fst, ust, pz, pb, colI, bins;   // float offsets
+    int flag;                                           // int offset: claimed item, ready flag
+    int ys;                                             // byte offset: characters of the chunk's columns
+    int bytes;
+};
+
+template <class SH, int T>
+__host__ __device__ inline SmemTeams make_smem_teams(int G) {
+    SmemTeams L;
+    int o = 0;
+    L.fst = o; o += T * ROWS * (2 * SH::SP + 4);
+    L.ust = o; o += T * ROWS * SH::KPP;
+    L.pz = o; o += T * TWT * 20;
+    L.pb = o; o += T * ROWS * (SH::NI + SH::ND);
+    L.colI = o; o += CRING * (SH::NI > 0 ? SH::NI : 1);
+    L.tM = o; o += al4(G * 441);
+    L.tI = o; o += al4(G * 21);
+    L.tD = o; o += al4(G * 21);
+    L.bins = o; o += al4(G * 21);
+    L.flag = o; o += 4;
+    L.ys = 4 * o;
+    L.bytes = L.ys + ((ROWS + CCH + 8 + 15) & ~15);
+    return L;
+}
+
+// quads [Q0, Q1) of a cell's record
+template <int Q0, int Q1, int N>
+__device__ __forceinline__ void load_row(float4 (&out)[N], const float *rec) {
+    const float4 *v = reinterpret_cast<const float4 *>(rec);
+#pragma unroll
+    for (int q = Q0; q < Q1; ++q) out[q] = v[q];
+}
+
+__device__ __forceinline__ void kahan(float &sum, float &comp, float v) {
+    const float y = v - comp, t = sum + y;
+    comp = (t - sum) - y;
+    sum = t;
+}
+
+// MK: a cell-masked batch (the stripes' live step ranges in P.srange)
+template <class SH, bool MK, int T>
+__device__ void count_chunk_teams(const KParams &P, int p, int si, int ch, const SmemTeams &L, float *sm,
+                               unsigned char *smb) {
+    constexpr int NE = SH::NE, NSRC = SH::NSRC, SP = SH::SP, KP = SH::KP, NM = SH::NM, NI = SH::NI;
+    constexpr int ND = SH::ND, KPP = SH::KPP, FS = 2 * SP + 4, NB4 = (NE + 3) / 4;
+    constexpr int THREADS = T * TWT;
+    constexpr int GROUPS64 = TWT / SH::NBLK;   // row groups of the outer products over 64 threads
+    constexpr int Q = 16 / T;                  // compensated sums of a thread (its team's 64 x 16 over T teams)
+    constexpr int NCD = (ROWS * ND + THREADS - 1) / THREADS;
+    static_assert(T == 1 || T == 2 || T == 4, "sums of a thread are whole float4s");
+    const PairMeta m = P.meta[p];
+    const int N = P.N, G = P.G;
+    const int Lx = m.Lx, Ly = m.Ly;
+    const int tid = threadIdx.x, team = tid / TWT, r = tid % TWT;
+    const int i0 = si * ROWS;
+    const int nrows = min(ROWS, Lx + 1 - i0);
+    const bool has_below = si + 1 < m.n_stripes;
+    const int64_t latc = m.lat_base + (int64_t)si * (ROWS + Ly) * ROWS;
+    const int64_t latb = m.lat_base + (int64_t)(si + 1) * (ROWS + Ly) * ROWS;   // stripe below (row 0)
+    const int T_last = (nrows - 1) + Ly;
+    // under a cell mask the recursions visited only the steps [t_beg, t_last]
+    // of this stripe and columns [blo, bhi] of the first row below: the count
+    // covers those steps of the chunk and reads the rest as zero
+    int t_beg = 0, t_last = T_last, blo = 0, bhi = Ly;
+    if (MK) {
+        const int2 rg = P.srange[m.stripe_base + si];
+        t_beg = max(0, rg.x);
+        t_last = min(T_last, rg.y + nrows - 1);
+        if (has_below) {
+            const int2 rb = P.srange[m.stripe_base + si + 1];
+            blo = max(0, rb.x);
+            bhi = min(Ly, rb.y);
+        }
+    }
+    const int t_hi = min(t_last, ch * CCH + CCH - 1);
+    const int t_lo = max(ch * CCH, t_beg);
+    if (t_lo > t_hi) return;                    // uniform over the CTA
+    int *s_flag = reinterpret_cast<int *>(sm) + L.flag + 1;
+    if (P.count_wait) {   // the wavefronts may still run: wait for the stripes read here
+        if (tid == 0) *s_flag = count_ready(P, m, si) ? 1 : 0;
+        __syncthreads();
+        const int ok = *s_flag;
+        __syncthreads();
+        if (!ok) {
+            if (tid == 0) atomicOr(P.status + p, PHMM_ST_TIMEOUT);
+            return;
+        }
+    }
+    const double llv = __ldcg(P.ll + p);
+    if (!(llv > -1e29)) return;   // uniform over the CTA
+    const double lam = llv / LN2;
+    const double Epd = floor(lam);
+    const int Ep = (int)Epd;
+    const float rfrac = (float)exp2(-(lam - Epd));
+    const int rowi = i0 + r;
+
+    // ---- the cell (t, r): its record and its successors', in flight or there
+    float4 fv[SP / 4], bv[NB4], sv[NB4], sd[NB4];   // sv: I types of (i, j+1), M types of (i+1, j+1); sd: D types of (i+1, j)
+    float4 svm[(NM + 3) / 4 > 0 ? (NM + 3) / 4 : 1];
+    int Ef = EXP_NONE, Eb = EXP_NONE, EI = EXP_NONE, ED = EXP_NONE, EM = EXP_NONE;
+    auto load_cell = [&](int t) {
+        Ef = Eb = EI = ED = EM = EXP_NONE;
+        const int jc = t - r;
+        if (t < t_lo || r >= nrows || jc < 0 || jc > Ly) return;
+        const int64_t c = latc + (int64_t)t * ROWS + r;
+        Ef = P.lat_exp[c];
+        Eb = P.blat_exp[c];
+        load_row<0, SP / 4>(fv, P.lat + c * SP);
+        load_row<0, NB4>(bv, P.blat + c * SP);
+        if (jc < Ly && (!MK || t + 1 <= t_last)) {
+            EI = P.blat_exp[c + ROWS];
+            load_row<NM / 4, (NM + NI + 3) / 4>(sv, P.blat + (c + ROWS) * SP);
+        }
+        if (rowi < Lx) {   // the row below: of this stripe, or the first of the next
+            const bool in = r + 1 < ROWS;
+            if (in ? (!MK || t + 1 <= t_last) : (!MK || (jc >= blo && jc <= bhi))) {
+                const int64_t s = in ? c + ROWS + 1 : latb + (int64_t)jc * ROWS;
+                ED = P.blat_exp[s];
+                load_row<(NM + NI) / 4, NB4>(sd, P.blat + s * SP);
+            }
+            if (jc < Ly && (in ? (!MK || t + 2 <= t_last) : (!MK || (jc + 1 >= blo && jc + 1 <= bhi)))) {
+                const int64_t s = in ? c + 2 * ROWS + 1 : latb + (int64_t)(jc + 1) * ROWS;
+                EM = P.blat_exp[s];
+                load_row<0, (NM + 3) / 4>(svm, P.blat + s * SP);
+            }
+        }
+    };
+    load_cell(t_hi - team);
+
+    // ---- tables, y characters of the chunk's columns, zeroed bins and columns
+    const int ybase = max(0, t_lo - (ROWS - 1));
+    unsigned char *ys = smb + L.ys;
+    {
+        const float *eM = P.eM + (int64_t)p * P.eM_stride;
+        const float *eI = P.eI + (int64_t)p * P.eID_stride;
+        const float *eDg = P.eD + (int64_t)p * P.eID_stride;
+        for (int idx = tid; idx < G * 441; idx += THREADS) sm[L.tM + idx] = __ldg(eM + idx);
+        for (int idx = tid; idx < G * 21; idx += THREADS) {
+            sm[L.tI + idx] = __ldg(eI + idx);
+            sm[L.tD + idx] = __ldg(eDg + idx);
+            sm[L.bins + idx] = 0.f;
+        }
+        for (int j = ybase + tid; j <= min(Ly, t_hi + 1); j += THREADS)
+            ys[j - ybase] = (unsigned char)(j >= 1 ? min((int)P.res[m.y_off + j - 1], 20) : 0);
+        for (int idx = tid; idx < CRING * NI; idx += THREADS) sm[L.colI + idx] = 0.f;
+        __syncthreads();
+    }
+    const int xch = row_char(P, p, m, rowi), xsucc = row_char(P, p, m, rowi + 1);
+    float eD[ND > 0 ? ND : 1];
+#pragma unroll
+    for (int k = 0; k < ND; ++k) eD[k] = sm[L.tD + P.w_group[NM + NI + k] * 21 + xsucc];
+    double *cntM_pair = P.cntM + (int64_t)p * G * 441 + xch * 21;
+
+    const int blk = r % SH::NBLK, grp = r / SH::NBLK;
+    const bool counter = grp < GROUPS64;
+    const int bs = blk / SH::BK, bk = blk % SH::BK;
+    // this thread's sums: Q of the 16 of thread `own` of every team; NCD of the D posteriors
+    const int own = tid / T, part = tid % T;
+    float csum[Q], ccomp[Q], dcnt[NCD > 0 ? NCD : 1], dcmp[NCD > 0 ? NCD : 1];
+#pragma unroll
+    for (int u = 0; u < Q; ++u) { csum[u] = 0.f; ccomp[u] = 0.f; }
+#pragma unroll
+    for (int k = 0; k < NCD; ++k) { dcnt[k] = 0.f; dcmp[k] = 0.f; }
+    // the I posteriors of the columns completed by the round at step tp move to the bins
+    auto finish_columns = [&](int tp, int n) {
+        for (int g = tid; g < G; g += THREADS)
+            for (int j = min(tp, Ly); j > tp - n; --j) {
+                if (j < 0) break;
+                float *col = sm + L.colI + (j & (CRING - 1)) * NI;
+                float &bin = sm[L.bins + g * 21 + ys[j - ybase]];
+#pragma unroll
+                for (int k = 0; k < NI; ++k)
+                    if (P.w_group[NM + k] == g) {
+                        bin += col[k];
+                        col[k] = 0.f;
+                    }
+            }
+    };
+
+    int n_prev = 0;
+    for (int tt = t_hi; tt >= t_lo; tt -= T) {
+        const int n = min(T, tt - t_lo + 1), t = tt - team;   // steps of this round
+        if (team < n) {
+            const int jc = t - r;
+            const bool valid = r < nrows && jc >= 0 && jc <= Ly;
+            const bool term = valid && rowi == Lx && jc == Ly;
+            float fsc = 0.f;
+            if (valid && Ef > EXP_NONE && Eb > EXP_NONE) {
+                int d = Ef + Eb - Ep;
+                if (d > 126) { d = 126; atomicOr(P.status + p, PHMM_ST_SCALE_CLAMP); }
+                fsc = scale_pow2(rfrac, max(d, -200));
+            }
+            const bool live = fsc > 0.f;
+            float ft[SP];
+#pragma unroll
+            for (int q = 0; q < SP / 4; ++q) {
+                const float va[4] = {fv[q].x, fv[q].y, fv[q].z, fv[q].w};
+#pragma unroll
+                for (int u = 0; u < 4; ++u) ft[4 * q + u] = (4 * q + u < NSRC && live) ? va[u] * fsc : 0.f;
+            }
+            float4 *fd = reinterpret_cast<float4 *>(sm + L.fst + (team * ROWS + r) * FS);
+#pragma unroll
+            for (int q = 0; q < SP / 2; ++q) fd[q] = make_float4(ft[2 * q], ft[2 * q], ft[2 * q + 1], ft[2 * q + 1]);
+            // u~[k] = w~_succ(k)[k] * 2^(E_succ - Eb)
+            const float uM = (live && EM > EXP_NONE) ? fminf(scale_pow2(1.f, EM - Eb), 3e38f) : 0.f;
+            const float uI = (live && EI > EXP_NONE) ? fminf(scale_pow2(1.f, EI - Eb), 3e38f) : 0.f;
+            const float uD = (live && ED > EXP_NONE) ? fminf(scale_pow2(1.f, ED - Eb), 3e38f) : 0.f;
+            const int ysu = (valid && jc < Ly) ? ys[jc + 1 - ybase] : 0;
+            float uk[KP];
+#pragma unroll
+            for (int k = 0; k < KP; ++k) {
+                float u = 0.f;
+                if (k < NE) {
+                    const int ty = SH::type_of(k);
+                    const float4 v4 = ty == T_M ? svm[k / 4] : (ty == T_I ? sv[k / 4] : sd[k / 4]);
+                    const float w = (k & 3) == 0 ? v4.x : ((k & 3) == 1 ? v4.y : ((k & 3) == 2 ? v4.z : v4.w));
+                    if (ty == T_M) u = uM > 0.f ? (w * sm[L.tM + P.w_group[k] * 441 + xsucc * 21 + ysu]) * uM : 0.f;
+                    else if (ty == T_I) u = uI > 0.f ? (w * sm[L.tI + P.w_group[k] * 21 + ysu]) * uI : 0.f;
+                    else u = uD > 0.f ? (w * eD[k - NM - NI]) * uD : 0.f;
+                }
+                uk[k] = u;
+            }
+            float4 *ud = reinterpret_cast<float4 *>(sm + L.ust + (team * ROWS + r) * KPP);
+#pragma unroll
+            for (int q = 0; q < KP / 4; ++q) ud[q] = make_float4(uk[4 * q], uk[4 * q + 1], uk[4 * q + 2], uk[4 * q + 3]);
+            const int yj = valid ? ys[jc - ybase] : 0;
+#pragma unroll
+            for (int k = 0; k < NE; ++k) {
+                const int ty = SH::type_of(k);
+                const float4 b4 = bv[k / 4];
+                const float b = (k & 3) == 0 ? b4.x : ((k & 3) == 1 ? b4.y : ((k & 3) == 2 ? b4.z : b4.w));
+                if (ty == T_M) {
+                    const float pk = live ? ft[k] * b : 0.f;
+                    if (pk != 0.f) atomicAdd(cntM_pair + P.w_group[k] * 441 + yj, (double)pk);
+                } else {   // -1: nothing to add
+                    sm[L.pb + (team * ROWS + r) * (NI + ND) + k - NM] = live ? b : -1.f;
+                }
+            }
+            if (term && live) {   // expected End transitions
+#pragma unroll
+                for (int s = 0; s < NSRC; ++s) {
+                    const float4 b4 = reinterpret_cast<const float4 *>(P.blat + (latc + (int64_t)t * ROWS + r) * SP)[s / 4];
+                    const float bs_ = (s & 3) == 0 ? b4.x : ((s & 3) == 1 ? b4.y : ((s & 3) == 2 ? b4.z : b4.w));
+                    atomicAdd(P.n_trans + ((int64_t)p * N + P.w_orig[s]) * N + P.e_idx, (double)(ft[s] * bs_));
+                }
+            }
+        }
+        load_cell(t - T);
+        __syncthreads();   // the round's f~, u~ and staged posteriors are there
+        if (n_prev) finish_columns(tt + T, n_prev);
+        if (team < n && counter) {
+            float2 pz[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) pz[u] = make_float2(0.f, 0.f);
+            const float4 *fb = reinterpret_cast<const float4 *>(sm + L.fst + team * ROWS * FS) + 2 * bs;
+            const float4 *ub = reinterpret_cast<const float4 *>(sm + L.ust + team * ROWS * KPP) + bk;
+            auto row_outer = [&](int rr) {
+                const float4 f0 = fb[rr * (FS / 4)], f1 = fb[rr * (FS / 4) + 1], u = ub[rr * (KPP / 4)];
+                const float2 ul = make_float2(u.x, u.y), uh = make_float2(u.z, u.w);
+                const float2 fa[4] = {make_float2(f0.x, f0.y), make_float2(f0.z, f0.w), make_float2(f1.x, f1.y),
+                                      make_float2(f1.z, f1.w)};
+#pragma unroll
+                for (int a = 0; a < 4; ++a) {
+                    pz[2 * a] = __ffma2_rn(fa[a], ul, pz[2 * a]);
+                    pz[2 * a + 1] = __ffma2_rn(fa[a], uh, pz[2 * a + 1]);
+                }
+            };
+            if constexpr (ROWS % GROUPS64 == 0) {
+                constexpr int RPG = ROWS / GROUPS64;
+                const int r0 = grp * RPG;
+#pragma unroll 4
+                for (int rr = r0; rr < r0 + RPG; ++rr) row_outer(rr);
+            } else {
+                const int r0 = grp * ROWS / GROUPS64, r1 = (grp + 1) * ROWS / GROUPS64;
+                for (int rr = r0; rr < r1; ++rr) row_outer(rr);
+            }
+            float4 *z = reinterpret_cast<float4 *>(sm + L.pz + (team * TWT + r) * 20);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) z[q] = make_float4(pz[2 * q].x, pz[2 * q].y, pz[2 * q + 1].x, pz[2 * q + 1].y);
+        }
+        __syncthreads();   // the partial products are there
+        if (own < GROUPS64 * SH::NBLK) {
+            for (int i = 0; i < n; ++i) {
+                const float4 *z = reinterpret_cast<const float4 *>(sm + L.pz + (i * TWT + own) * 20) + part * (Q / 4);
+#pragma unroll
+                for (int q = 0; q < Q / 4; ++q) {
+                    const float4 v = z[q];
+                    kahan(csum[4 * q], ccomp[4 * q], v.x);
+                    kahan(csum[4 * q + 1], ccomp[4 * q + 1], v.y);
+                    kahan(csum[4 * q + 2], ccomp[4 * q + 2], v.z);
+                    kahan(csum[4 * q + 3], ccomp[4 * q + 3], v.w);
+                }
+            }
+        }
+        // D and I posteriors f~ b~ (each rounded once, in its sum)
+        const float *fs = sm + L.fst, *pb = sm + L.pb;
+        for (int i = 0; i < n; ++i) {
+#pragma unroll
+            for (int k = 0; k < NCD; ++k) {
+                const int c = tid + k * THREADS, row = i * ROWS + c / ND, kd = NI + c % ND;
+                const float b = c < ROWS * ND ? pb[row * (NI + ND) + kd] : -1.f;
+                if (b != -1.f) {
+                    const float y = fmaf(fs[row * FS + 2 * (NM + kd)], b, -dcmp[k]), s = dcnt[k] + y;
+                    dcmp[k] = (s - dcnt[k]) - y;
+                    dcnt[k] = s;
+                }
+            }
+        }
+        // column j takes row tt - i - j of each of the round's steps
+        for (int c = tid; c < (ROWS + T - 1) * NI; c += THREADS) {
+            const int j = tt - (ROWS - 1) - (T - 1) + c / NI, k = c % NI;
+            if (j < 0 || j > Ly) continue;
+            float *col = sm + L.colI + (j & (CRING - 1)) * NI + k;
+            float v = *col;
+#pragma unroll
+            for (int i = 0; i < T; ++i) {
+                const int row = tt - i - j;
+                if (i < n && row >= 0 && row < ROWS) {
+                    const float b = pb[(i * ROWS + row) * (NI + ND) + k];
+                    if (b != -1.f) v = fmaf(fs[(i * ROWS + row) * FS + 2 * (NM + k)], b, v);
+                }
+            }
+            *col = v;
+        }
+        n_prev = n;
+        __syncthreads();   // the next round writes all of it again
+    }
+    // ---- flush the chunk's partial counts (float64 reductions)
+    finish_columns(t_lo + n_prev - 1, n_prev);
+    if (own < GROUPS64 * SH::NBLK) {
+        float *z = sm + L.pz + own * 20 + part * Q;
+#pragma unroll
+        for (int u = 0; u < Q; ++u) z[u] = csum[u] - ccomp[u];
+    }
+#pragma unroll
+    for (int k = 0; k < NCD; ++k) {
+        const int c = tid + k * THREADS;
+        if (c >= ROWS * ND) continue;
+        const int row = c / ND, kd = c % ND;
+        const float v = dcnt[k] - dcmp[k];
+        if (row < nrows && i0 + row >= 1 && v != 0.f)
+            atomicAdd(P.cntD + ((int64_t)p * G + P.w_group[NM + NI + kd]) * 21 + row_char(P, p, m, i0 + row), (double)v);
+    }
+    __syncthreads();
+    // n_trans: the row groups' sums of an entry in float64, then one addition
+    // for the entry (several where the entries are fewer than the threads)
+    {
+        constexpr int C = SH::NBLK * 16, SL = C < THREADS ? (THREADS / C < GROUPS64 ? THREADS / C : GROUPS64) : 1;
+        const float *chi = P.chi + (int64_t)p * P.chi_stride;
+        for (int c = tid; c < C * SL; c += THREADS) {
+            const int u = c % 16, b = (c / 16) % SH::NBLK, sl = c / C;
+            const int s = 4 * (b / SH::BK) + (u >> 2), k = 4 * (b % SH::BK) + (u & 3);
+            if (s >= NSRC || k >= NE) continue;
+            double v = 0.0;
+            for (int g = sl; g < GROUPS64; g += SL) v += (double)sm[L.pz + (g * SH::NBLK + b) * 20 + u];
+            if (v == 0.0) continue;
+            const int os = P.w_orig[s], ok = P.w_orig[k];
+            atomicAdd(P.n_trans + ((int64_t)p * N + os) * N + ok, v * (double)__ldg(chi + os * N + ok));
+        }
+    }
+    // I-type columns not completed inside the chunk (touched by rows below row 0)
+    for (int c = tid; c < (ROWS - 1) * NI; c += THREADS) {
+        const int j = t_lo - (ROWS - 1) + c / NI, k = c % NI;
+        if (j < 0 || j > Ly) continue;
+        const float v = sm[L.colI + (j & (CRING - 1)) * NI + k];
+        if (v != 0.f) atomicAdd(P.cntI + ((int64_t)p * G + P.w_group[NM + k]) * 21 + ys[j - ybase], (double)v);
+    }
+    for (int idx = tid; idx < G * 21; idx += THREADS) {
+        const float v = sm[L.bins + idx];
+        if (v != 0.f) atomicAdd(P.cntI + (int64_t)p * G * 21 + idx, (double)v);
+    }
+    __syncthreads();
+}
+
+template <class SH, bool MK, int T>
+__global__ void __launch_bounds__(T *TWT, SH::SP > 16 ? 1 : 2) count_teams_kernel(const KParams P) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    float *sm = reinterpret_cast<float *>(smem_raw);
+    const SmemTeams L = make_smem_teams<SH, T>(P.G);
+    int *s_item = reinterpret_cast<int *>(sm) + L.flag;
+    for (;;) {
+        if (threadIdx.x == 0) *s_item = count_claim(P);
+        __syncthreads();
+        const int it = *s_item;
+        __syncthreads();
+        if (it >= P.n_items) break;
+        const int2 w = P.items[it];
+        count_chunk_teams<SH, MK, T>(P, w.x, w.y >> 12, w.y & 4095, L, sm, smem_raw);
+    }
+}
+
+}  // namespace warp2
