@@ -270,6 +270,7 @@ __global__ void __launch_bounds__(32 * SH::NB) fwdbwd_block_kernel(const KParams
 // ---------------------------------------------------------------- counts from both lattices
 struct SmemCB {
     int tM, tI, tD, fst, ust, rowM, rowD, colI, binsI;   // float offsets
+    int eoff, klist;                                    // int16 offsets (in 2-byte units): see count_chunk_b
     int ys;                                             // byte offset
     int bytes;
 };
@@ -278,7 +279,7 @@ struct SmemCB {
 // mod 64][I slot], D: [row][D slot]): a cell's slots are owned by one thread
 // each and the cells of one step have distinct rows and columns, so the bins
 // need no atomics.  wM / wI / wD are the slot widths of the three types.
-__host__ __device__ inline SmemCB make_smem_cb(int NS, int G, int max_ly, int wM, int wI, int wD) {
+__host__ __device__ inline SmemCB make_smem_cb(int NS, int G, int wM, int wI, int wD) {
     const int SPR = spr_of(NS);
     SmemCB L;
     int o = 0;
@@ -291,34 +292,21 @@ __host__ __device__ inline SmemCB make_smem_cb(int NS, int G, int max_ly, int wM
     L.rowD = o; o += al4(ROWS * wD);
     L.colI = o; o += al4(ROWS * wI);
     L.binsI = o; o += al4(G * 21);
+    L.eoff = 2 * o; o += al4((NS + 1) / 2);
+    L.klist = 2 * o; o += al4((G * wI + 1) / 2);
     int bytes = o * 4;
     L.ys = bytes;
-    bytes += max_ly + 2;
+    bytes += ROWS + CCHB + 8;   // the characters of the chunk's columns
     L.bytes = (bytes + 15) & ~15;
     return L;
 }
 
-// emission factors of the 4 slots of quad q at characters (xi, yj)
-__device__ __forceinline__ float4 quad_emit_at(const KParams &P, const float *sm, const SmemCB &L, int q, int xi, int yj) {
-    float v[4];
-    const int qt = P.quad_type[q];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-        const int k = 4 * q + u;
-        const int kt = P.slot_type[k];
-        const bool em = (kt == T_M || kt == T_I || kt == T_D);
-        const int g = em ? P.slot_group[k] : 0;
-        float e = 0.f;
-        if (em) {
-            if (qt == T_M) e = sm[L.tM + g * 441 + xi * 21 + yj];
-            else if (qt == T_I) e = sm[L.tI + g * 21 + yj];
-            else e = sm[L.tD + g * 21 + xi];
-        }
-        v[u] = e;
-    }
-    return make_float4(v[0], v[1], v[2], v[3]);
-}
-
+// What a thread needs of its quads' types, groups and places is looked up once a
+// chunk, not once a step: by slot out of the kernel's parameters (indexed constant loads,
+// one a lane group), with a branch a slot and the I-type bins by one thread, a step took
+// 1780 instructions a warp, two thirds of them outside the outer products
+// (32 pairs of 200-1500 at 42 states: 7.86 ms; now 5.98 ms, 1150 a warp, and shared-memory
+// wavefronts at 63 % of their peak).
 template <class SH>
 __device__ void count_chunk_b(const KParams &P, int p, int si, int ch, const SmemCB &L, float *sm, unsigned char *smb) {
     constexpr int NS = SH::NS, NB = SH::NB, NBP = SH::NBP, SPR = SH::SPR;
@@ -354,6 +342,7 @@ __device__ void count_chunk_b(const KParams &P, int p, int si, int ch, const Sme
     const float rfrac = (float)exp2(-(lam - floor(lam)));
     const int mb = P.kbeg[0], ib = P.kbeg[1], db = P.kbeg[2];
     const int wM = P.kend[0] - mb, wI = P.kend[1] - ib, wD = P.kend[2] - db;
+    const int jlo = max(0, t0 - (ROWS - 1));
     {
         const float *eM = P.eM + (int64_t)p * P.eM_stride;
         const float *eI = P.eI + (int64_t)p * P.eID_stride;
@@ -367,18 +356,31 @@ __device__ void count_chunk_b(const KParams &P, int p, int si, int ch, const Sme
         for (int idx = tid; idx < ROWS * wM * 21; idx += CNT_THREADS) sm[L.rowM + idx] = 0.f;
         for (int idx = tid; idx < ROWS * wD; idx += CNT_THREADS) sm[L.rowD + idx] = 0.f;
         for (int idx = tid; idx < ROWS * wI; idx += CNT_THREADS) sm[L.colI + idx] = 0.f;
+        // slot -> offset of its group in the table of its type (-1: the start, padding)
+        for (int s = tid; s < NS; s += CNT_THREADS) {
+            const int st = P.slot_type[s];
+            reinterpret_cast<int16_t *>(sm)[L.eoff + s] = (int16_t)(
+                st == T_M ? P.slot_group[s] * 441 : ((st == T_I || st == T_D) ? P.slot_group[s] * 21 : -1));
+        }
         unsigned char *ysw = smb + L.ys;
-        const int jlo = max(0, t0 - (ROWS - 1)), jhi = min(Ly, t_hi + 1);
+        const int jhi = min(Ly, t_hi + 1);
         for (int j = jlo + tid; j <= jhi; j += CNT_THREADS) {
             int c = 0;
             if (j >= 1) c = min((int)P.res[m.y_off + j - 1], 20);
-            ysw[j] = (unsigned char)c;
+            ysw[j - jlo] = (unsigned char)c;
         }
     }
     __syncthreads();
-    const unsigned char *ys = smb + L.ys;
+    const unsigned char *ys = smb + L.ys - jlo;
     float *fst = sm + L.fst, *ust = sm + L.ust;
     float *rowM = sm + L.rowM, *rowD = sm + L.rowD, *colI = sm + L.colI, *binsI = sm + L.binsI;
+    // the I-type slots of a group, for the thread that adds them to its bins
+    const int gI = CNT_THREADS - 1 - tid;   // (threads without an outer-product tile, where there are any)
+    int16_t *klist = reinterpret_cast<int16_t *>(sm) + L.klist + gI * wI;
+    int nI = 0;
+    if (gI < G)
+        for (int k = 0; k < wI; ++k)
+            if (P.slot_type[ib + k] == T_I && P.slot_group[ib + k] == gI) klist[nI++] = (int16_t)k;
     // phase A role: cell row rho, quads sub, sub+4, ...
     const int rho = tid >> 2, sub = tid & 3;
     const int irow = i0 + rho;
@@ -398,6 +400,23 @@ __device__ void count_chunk_b(const KParams &P, int p, int si, int ch, const Sme
 #pragma unroll
         for (int u = 0; u < 16; ++u) { csum[a][u] = 0.f; ccomp[a][u] = 0.f; }
 
+    // this thread's quads: type, emission table entry of the successor's row, emission bins
+    int qt[QPT], ebase[QPT], sdelta[QPT];
+    float *acc[QPT];
+#pragma unroll
+    for (int a = 0; a < QPT; ++a) {
+        const int q = sub + 4 * a;
+        qt[a] = q < NB ? (int)P.quad_type[q] : T_NONE;
+        ebase[a] = qt[a] == T_M ? L.tM + xn * 21 : (qt[a] == T_I ? L.tI : L.tD + xn);
+        sdelta[a] = qt[a] == T_M ? 2 * ROWS + 1 : (qt[a] == T_I ? ROWS : ROWS + 1);   // cells to the successor
+        acc[a] = qt[a] == T_M ? rowM + (rho * wM + 4 * q - mb) * 21
+                              : (qt[a] == T_I ? colI + 4 * q - ib : rowD + rho * wD + 4 * q - db);
+    }
+    const int16_t *eoff = reinterpret_cast<const int16_t *>(sm) + L.eoff + 4 * sub;
+    // the successors of the stripe's last row are the next stripe's first
+    const bool last_row = rho + 1 >= nrows;
+    const bool row_below = irow + 1 <= Lx && (!last_row || has_below);
+
     // lattice loads of one step for this thread's cell and quads; issued a step
     // ahead (before the outer products of the current step) so their latency
     // hides behind phase B
@@ -407,28 +426,29 @@ __device__ void count_chunk_b(const KParams &P, int p, int si, int ch, const Sme
         const int j = t - rho;
         const bool valid = t >= t0 && rho < nrows && j >= 0 && j <= Ly;
         const int64_t cell = latc + (int64_t)t * ROWS + rho;
-        const bool hI = j + 1 <= Ly, hD = irow + 1 <= Lx, hM = hI && hD;
+        const float *f = P.lat + cell * NS + 4 * sub, *b = P.blat + cell * NS + 4 * sub;
+        const int *fe = P.lat_exp + cell * NBP + sub, *be = P.blat_exp + cell * NBP + sub;
 #pragma unroll
         for (int a = 0; a < QPT; ++a) {
-            const int q = sub + 4 * a;
             Ef[a] = EXP_NONE; Eb[a] = EXP_NONE; Es[a] = EXP_NONE;
             fv[a] = make_float4(0.f, 0.f, 0.f, 0.f); bv[a] = fv[a]; sv[a] = fv[a];
-            if (!valid || q >= NB) continue;
+            if (!valid || sub + 4 * a >= NB) continue;
             // every quad of a valid cell is written (zero values with EXP_NONE)
-            Ef[a] = __ldcg(P.lat_exp + cell * NBP + q);
-            Eb[a] = __ldcg(P.blat_exp + cell * NBP + q);
-            fv[a] = __ldcg(reinterpret_cast<const float4 *>(P.lat + cell * NS) + q);
-            bv[a] = __ldcg(reinterpret_cast<const float4 *>(P.blat + cell * NS) + q);
-            const int qt = P.quad_type[q];
-            int64_t sc = -1;
-            if (qt == T_I && hI) sc = latc + (int64_t)(t + 1) * ROWS + rho;
-            else if (qt == T_D && hD && (rho + 1 < nrows || has_below))
-                sc = rho + 1 < nrows ? latc + (int64_t)(t + 1) * ROWS + rho + 1 : latb + (int64_t)j * ROWS;
-            else if (qt == T_M && hM && (rho + 1 < nrows || has_below))
-                sc = rho + 1 < nrows ? latc + (int64_t)(t + 2) * ROWS + rho + 1 : latb + (int64_t)(j + 1) * ROWS;
-            if (sc >= 0) {
-                Es[a] = __ldcg(P.blat_exp + sc * NBP + q);
-                sv[a] = __ldcg(reinterpret_cast<const float4 *>(P.blat + sc * NS) + q);
+            Ef[a] = __ldcg(fe + 4 * a);
+            Eb[a] = __ldcg(be + 4 * a);
+            fv[a] = __ldcg(reinterpret_cast<const float4 *>(f + 16 * a));
+            bv[a] = __ldcg(reinterpret_cast<const float4 *>(b + 16 * a));
+            const bool there = qt[a] == T_I ? j < Ly : (row_below && (qt[a] == T_D || (qt[a] == T_M && j < Ly)));
+            if (there) {
+                const float *sp = b + sdelta[a] * NS;
+                const int *se = be + sdelta[a] * NBP;
+                if (qt[a] != T_I && last_row) {
+                    const int64_t c = latb + (int64_t)(qt[a] == T_M ? j + 1 : j) * ROWS;
+                    sp = P.blat + c * NS + 4 * sub;
+                    se = P.blat_exp + c * NBP + sub;
+                }
+                Es[a] = __ldcg(se + 4 * a);
+                sv[a] = __ldcg(reinterpret_cast<const float4 *>(sp + 16 * a));
             }
         }
     };
@@ -454,37 +474,45 @@ __device__ void count_chunk_b(const KParams &P, int p, int si, int ch, const Sme
                 float4 ft = make_float4(0.f, 0.f, 0.f, 0.f), uu = ft;
                 if (live) {
                     if (Ef[a] > EXP_NONE) ft = f4scale(fv[a], pow2n(Ef[a] - Efm));
-                    // posteriors of my quad -> emission counts, End transitions
+                    // posteriors of my quad -> emission counts, End transitions (the start's and the
+                    // padding's bins are not read)
                     if (Eb[a] > EXP_NONE) {
                         int dp = Eb[a] + Efm - Ep;
                         if (dp > 126) { dp = 126; atomicOr(P.status + p, PHMM_ST_SCALE_CLAMP); }
                         const float ps = warp2::scale_pow2(rfrac, max(dp, -200));
                         const float pk[4] = {ft.x * bv[a].x * ps, ft.y * bv[a].y * ps, ft.z * bv[a].z * ps,
                                              ft.w * bv[a].w * ps};
+                        if (qt[a] == T_M) {
+                            float *m = acc[a] + yj;
 #pragma unroll
-                        for (int u = 0; u < 4; ++u) {
-                            const int s = 4 * q + u;
-                            const int st = P.slot_type[s];
-                            const float pv = pk[u];
-                            if (pv == 0.f) continue;
-                            if (st == T_M) rowM[(rho * wM + s - mb) * 21 + yj] += pv;
-                            else if (st == T_I) colI[(j % ROWS) * wI + s - ib] += pv;
-                            else if (st == T_D) rowD[rho * wD + s - db] += pv;
-                            if (term && P.slot_orig[s] >= 0)
-                                atomicAdd(P.n_trans + ((int64_t)p * N + P.slot_orig[s]) * N + P.e_idx, (double)pv);
+                            for (int u = 0; u < 4; ++u) m[21 * u] += pk[u];
+                        } else if (qt[a] != T_NONE) {
+                            float4 *c = reinterpret_cast<float4 *>(acc[a] + (qt[a] == T_I ? (j % ROWS) * wI : 0));
+                            float4 v = *c;
+                            v.x += pk[0];
+                            v.y += pk[1];
+                            v.z += pk[2];
+                            v.w += pk[3];
+                            *c = v;
+                        }
+                        if (term) {
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) {
+                                const int os = P.slot_orig[4 * q + u];
+                                if (os >= 0 && pk[u] != 0.f)
+                                    atomicAdd(P.n_trans + ((int64_t)p * N + os) * N + P.e_idx, (double)pk[u]);
+                            }
                         }
                     }
                     // successor operand of my destination quad
                     if (Es[a] > EXP_NONE && !term) {
-                        const int qt = P.quad_type[q];
-                        const int xi = qt == T_I ? xc : xn;
-                        const int yy = qt == T_D ? yj : yn;
                         int du = Es[a] + Efm - Ep;
                         if (du > 126) { du = 126; atomicOr(P.status + p, PHMM_ST_SCALE_CLAMP); }
                         const float us = fminf(warp2::scale_pow2(rfrac, max(du, -200)), 3e38f);
-                        const float4 e4 = quad_emit_at(P, sm, L, q, xi, yy);
-                        uu = make_float4(sv[a].x * e4.x * us, sv[a].y * e4.y * us, sv[a].z * e4.z * us,
-                                         sv[a].w * e4.w * us);
+                        const short4 o = *reinterpret_cast<const short4 *>(eoff + 16 * a);
+                        const float *e = sm + ebase[a] + (qt[a] == T_D ? 0 : yn);
+                        uu = make_float4(sv[a].x * (o.x >= 0 ? e[o.x] : 0.f) * us, sv[a].y * (o.y >= 0 ? e[o.y] : 0.f) * us,
+                                         sv[a].z * (o.z >= 0 ? e[o.z] : 0.f) * us, sv[a].w * (o.w >= 0 ? e[o.w] : 0.f) * us);
                     }
                 }
                 *reinterpret_cast<float4 *>(fst + rho * SPR + 4 * q) = ft;
@@ -494,14 +522,14 @@ __device__ void count_chunk_b(const KParams &P, int p, int si, int ch, const Sme
         issue(t - 1);
         __syncthreads();
         // column t is complete once row 0 visited it: I-type bins
-        if (tid == 0 && t <= Ly) {
-            const int slot = t % ROWS;
-            const int yj = ys[t];
-            for (int k = 0; k < wI; ++k) {
-                const int s = ib + k;
-                if (P.slot_type[s] == T_I) binsI[P.slot_group[s] * 21 + yj] += colI[slot * wI + k];
-                colI[slot * wI + k] = 0.f;
+        if (gI < G && t <= Ly) {
+            float *col = colI + (t % ROWS) * wI;
+            float v = binsI[gI * 21 + ys[t]];
+            for (int n = 0; n < nI; ++n) {
+                v += col[klist[n]];
+                col[klist[n]] = 0.f;
             }
+            binsI[gI * 21 + ys[t]] = v;
         }
         // ================= phase B: outer products of the step's cells
 #pragma unroll
@@ -511,22 +539,24 @@ __device__ void count_chunk_b(const KParams &P, int p, int si, int ch, const Sme
             if (!role) continue;
             const int b_s = TPT > 1 ? bidx / NB : bs, b_k = TPT > 1 ? bidx % NB : bk;
             const int r0 = TPT > 1 ? 0 : grp * ROWS / GRP, r1 = TPT > 1 ? ROWS : (grp + 1) * ROWS / GRP;
-            float pz[16];
+            float2 pz[8];
 #pragma unroll
-            for (int u = 0; u < 16; ++u) pz[u] = 0.f;
+            for (int u = 0; u < 8; ++u) pz[u] = make_float2(0.f, 0.f);
+#pragma unroll 4
             for (int rr = r0; rr < r1; ++rr) {
                 const float4 fv = *reinterpret_cast<const float4 *>(fst + rr * SPR + 4 * b_s);
                 const float4 uv = *reinterpret_cast<const float4 *>(ust + rr * SPR + 4 * b_k);
                 const float fa[4] = {fv.x, fv.y, fv.z, fv.w};
-                const float ua[4] = {uv.x, uv.y, uv.z, uv.w};
+                const float2 ul = make_float2(uv.x, uv.y), uh = make_float2(uv.z, uv.w);
 #pragma unroll
-                for (int x = 0; x < 4; ++x)
-#pragma unroll
-                    for (int y = 0; y < 4; ++y) pz[4 * x + y] = fmaf(fa[x], ua[y], pz[4 * x + y]);
+                for (int x = 0; x < 4; ++x) {
+                    pz[2 * x] = __ffma2_rn(make_float2(fa[x], fa[x]), ul, pz[2 * x]);
+                    pz[2 * x + 1] = __ffma2_rn(make_float2(fa[x], fa[x]), uh, pz[2 * x + 1]);
+                }
             }
 #pragma unroll
             for (int u = 0; u < 16; ++u) {
-                const float y = pz[u] - ccomp[a][u];
+                const float y = (u & 1 ? pz[u / 2].y : pz[u / 2].x) - ccomp[a][u];
                 const float tt = csum[a][u] + y;
                 ccomp[a][u] = (tt - csum[a][u]) - y;
                 csum[a][u] = tt;
@@ -589,7 +619,7 @@ __global__ void __launch_bounds__(CNT_THREADS, 2) count_block_kernel(const KPara
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int s_item;
     float *sm = reinterpret_cast<float *>(smem_raw);
-    const SmemCB L = make_smem_cb(SH::NS, P.G, P.max_ly, P.kend[0] - P.kbeg[0], P.kend[1] - P.kbeg[1],
+    const SmemCB L = make_smem_cb(SH::NS, P.G, P.kend[0] - P.kbeg[0], P.kend[1] - P.kbeg[1],
                                   P.kend[2] - P.kbeg[2]);
     for (;;) {
         __syncthreads();

@@ -2224,7 +2224,7 @@ int launch_block(phmm_plan *plan, KParams &K, int n_items, int max_ly, int kind,
     void (*kern)(const KParams) = nullptr;
     int bytes = 0, threads = 0;
     if (kind == 3) {
-        bytes = blk::make_smem_cb(SH::NS, K.G, max_ly, K.kend[0] - K.kbeg[0], K.kend[1] - K.kbeg[1],
+        bytes = blk::make_smem_cb(SH::NS, K.G, K.kend[0] - K.kbeg[0], K.kend[1] - K.kbeg[1],
                                   K.kend[2] - K.kbeg[2]).bytes;
         kern = blk::count_block_kernel<SH>;
         threads = blk::CNT_THREADS;
