@@ -245,7 +245,8 @@ __device__ __forceinline__ void quad_contract2(const float *v0, const int *e0, c
     Eref1 = EXP_NONE;
 #pragma unroll
     for (int b = 0; b < NB; ++b) { Eref0 = max(Eref0, E0[b]); Eref1 = max(Eref1, E1[b]); }
-    float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f, c0 = 0.f, c1 = 0.f, c2 = 0.f, c3 = 0.f;
+    const float2 z2 = make_float2(0.f, 0.f);
+    float2 al = z2, ah = z2, cl = z2, ch = z2;   // pairs of destinations: one issue for two multiply-adds
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
         const float s0 = pow2n(E0[b] - Eref0), s1 = pow2n(E1[b] - Eref1);
@@ -263,12 +264,30 @@ __device__ __forceinline__ void quad_contract2(const float *v0, const int *e0, c
                 const float4 cv = chi4q[s * (NS / 4)];
                 k0 = cv.x; k1 = cv.y; k2 = cv.z; k3 = cv.w;
             }
-            a0 = fmaf(xs[i], k0, a0); a1 = fmaf(xs[i], k1, a1); a2 = fmaf(xs[i], k2, a2); a3 = fmaf(xs[i], k3, a3);
-            c0 = fmaf(ysv[i], k0, c0); c1 = fmaf(ysv[i], k1, c1); c2 = fmaf(ysv[i], k2, c2); c3 = fmaf(ysv[i], k3, c3);
+            const float2 kl = make_float2(k0, k1), kh = make_float2(k2, k3);
+            const float2 x2 = make_float2(xs[i], xs[i]), y2 = make_float2(ysv[i], ysv[i]);
+            al = __ffma2_rn(x2, kl, al); ah = __ffma2_rn(x2, kh, ah);
+            cl = __ffma2_rn(y2, kl, cl); ch = __ffma2_rn(y2, kh, ch);
         }
     }
-    o0 = make_float4(a0, a1, a2, a3);
-    o1 = make_float4(c0, c1, c2, c3);
+    o0 = make_float4(al.x, al.y, ah.x, ah.y);
+    o1 = make_float4(cl.x, cl.y, ch.x, ch.y);
+}
+
+// a boundary cell (NS values, NBP exponents) by the lanes of a warp, 16 bytes each: out of the ring,
+// and into the halo slot
+__device__ __forceinline__ void store_edge_warp(const float *v, const int *e, float *gv, int *ge, int NS, int NBP, int lane) {
+    for (int i = lane; i < (NS + NBP) / 4; i += 32) {
+        if (i < NS / 4) reinterpret_cast<float4 *>(gv)[i] = reinterpret_cast<const float4 *>(v)[i];
+        else reinterpret_cast<int4 *>(ge)[i - NS / 4] = reinterpret_cast<const int4 *>(e)[i - NS / 4];
+    }
+}
+__device__ __forceinline__ void load_edge_warp(float *v, int *e, const float *gv, const int *ge, int NS, int NBP, int lane) {
+    for (int i = lane; i < (NS + NBP) / 4; i += 32) {
+        if (i < NS / 4) cp_async16(v + 4 * i, gv + 4 * i);
+        else cp_async16(e + 4 * i - NS, ge + 4 * i - NS);
+    }
+    cp_commit();
 }
 
 __device__ __forceinline__ void copy_edge_cell(const float *v, const int *e, float *gv, int *ge, int NS, int NBP) {
@@ -325,7 +344,9 @@ __device__ void fwd_stripe_b(const KParams &P, int p, int si, const SmemB &L, fl
     }
     const int qt = P.quad_type[q];
     const int T_last = (nrows - 1) + Ly;
-    // halo pipeline state (thread 0 only)
+    // halo pipeline state (warp 0; progress by its lane 0).  One thread moving a boundary
+    // cell's 14 vectors in and 14 out a step (42 states) held its warp and the step's
+    // barrier (one pair of 511 x 600, forward: 2.52 ms; by the warp 2.38)
     int pv = 0, fetched = 0;   // columns [0, fetched) of the halo row are in flight or landed
     if (tid == 0) { misc[0] = 0; if (has_above) pv = ld_acquire(prog_above); }
     double llpart = 0.0;
@@ -333,17 +354,16 @@ __device__ void fwd_stripe_b(const KParams &P, int p, int si, const SmemB &L, fl
 
     for (int t = 0; t <= T_last; ++t) {
         // ---- halo column t (row i0-1) must be in shared memory before the step barrier
-        if (tid == 0 && has_above && t <= Ly) {
+        if (q == 0 && has_above && t <= Ly) {
             if (fetched <= t) {   // not prefetched: wait for the producer, fetch now
-                if (!wait_geq(prog_above, t + 1, P.spin_limit)) {
-                    misc[0] = 1;
+                int ok = 1;
+                if (lane == 0) ok = wait_geq(prog_above, t + 1, P.spin_limit) ? 1 : 0;
+                ok = __shfl_sync(0xffffffffu, ok, 0);
+                if (!ok) {
+                    if (lane == 0) misc[0] = 1;
                 } else {
-                    const int sl = t % 3;
-                    for (int i = 0; i < NS / 4; ++i)
-                        cp_async16(halo + sl * NS + 4 * i, edge_above + (int64_t)t * NS + 4 * i);
-                    for (int i = 0; i < NBP / 4; ++i)
-                        cp_async16(haloE + sl * NBP + 4 * i, edgeE_above + (int64_t)t * NBP + 4 * i);
-                    cp_commit();
+                    load_edge_warp(halo + (t % 3) * NS, haloE + (t % 3) * NBP, edge_above + (int64_t)t * NS,
+                                   edgeE_above + (int64_t)t * NBP, NS, NBP, lane);
                     fetched = t + 1;
                 }
             }
@@ -352,28 +372,29 @@ __device__ void fwd_stripe_b(const KParams &P, int p, int si, const SmemB &L, fl
         bar_sync(BAR_STEP, NB * 32);
         if (misc[0]) break;                       // uniform: written before the barrier
         // ---- bottom row of step t-1 (every warp wrote its quad before the barrier):
-        // thread 0 copies it to the edge row and publishes; its own release covers it
-        if (tid == 0 && has_below && t >= 1) {
+        // warp 0 copies it to the edge row, and its lane 0 publishes
+        if (q == 0 && has_below && t >= 1) {
             const int jb = t - 1 - (ROWS - 1);
             if (jb >= 0 && jb <= Ly) {
-                copy_edge_cell(ring + ((t + 2) % 3) * ROWS * SPR + (ROWS - 1) * SPR,
-                               ringE + ((t + 2) % 3) * ROWS * NBP + (ROWS - 1) * NBP,
-                               edge_mine + (int64_t)jb * NS, edgeE_mine + (int64_t)jb * NBP, NS, NBP);
-                if (((jb + 1) % PUBB) == 0 || jb == Ly) st_release(prog_mine, jb + 1);
+                store_edge_warp(ring + ((t + 2) % 3) * ROWS * SPR + (ROWS - 1) * SPR,
+                                ringE + ((t + 2) % 3) * ROWS * NBP + (ROWS - 1) * NBP,
+                                edge_mine + (int64_t)jb * NS, edgeE_mine + (int64_t)jb * NBP, NS, NBP, lane);
+                if (((jb + 1) % PUBB) == 0 || jb == Ly) {
+                    __threadfence();
+                    __syncwarp();
+                    if (lane == 0) st_release(prog_mine, jb + 1);
+                }
             }
         }
         // ---- prefetch halo column t+1 when the progress read at the last step covers it
-        if (tid == 0 && has_above && t + 1 <= Ly) {
-            if (fetched == t + 1 && pv > t + 1) {
-                const int sl = (t + 1) % 3;
-                for (int i = 0; i < NS / 4; ++i)
-                    cp_async16(halo + sl * NS + 4 * i, edge_above + (int64_t)(t + 1) * NS + 4 * i);
-                for (int i = 0; i < NBP / 4; ++i)
-                    cp_async16(haloE + sl * NBP + 4 * i, edgeE_above + (int64_t)(t + 1) * NBP + 4 * i);
-                cp_commit();
+        if (q == 0 && has_above && t + 1 <= Ly) {
+            const int sl = (t + 1) % 3;
+            if (__shfl_sync(0xffffffffu, (fetched == t + 1 && pv > t + 1) ? 1 : 0, 0)) {
+                load_edge_warp(halo + sl * NS, haloE + sl * NBP, edge_above + (int64_t)(t + 1) * NS,
+                               edgeE_above + (int64_t)(t + 1) * NBP, NS, NBP, lane);
                 fetched = t + 2;
             }
-            if (pv <= t + 2) pv = ld_acquire(prog_above);   // only when the next prefetch needs more
+            if (lane == 0 && pv <= t + 2) pv = ld_acquire(prog_above);   // only when the next prefetch needs more
         }
         // ---- my quad for both cells: predecessors, then one merged contraction
         const float *pvp[R];
@@ -464,7 +485,7 @@ __device__ void fwd_stripe_b(const KParams &P, int p, int si, const SmemB &L, fl
             atomicOr(P.status + p, PHMM_ST_TIMEOUT);
             if (si + 1 == m.n_stripes) P.ll[p] = NEG_INF_LL;
         }
-        if (tid == 0) cp_wait0();
+        if (q == 0) cp_wait0();
         __threadfence();
         bar_sync(BAR_STEP, NB * 32);
         if (tid == 0) st_release(P.progress + m.stripe_base + si, Ly + 2);
@@ -500,8 +521,9 @@ __device__ void fwd_stripe_b(const KParams &P, int p, int si, const SmemB &L, fl
     if (tid == 0) st_release(P.progress + m.stripe_base + si, Ly + 2);
 }
 
-template <class SH>
-__global__ void __launch_bounds__(32 * SH::NB) forward_block_kernel(const KParams P) {
+// PER_SM: CTAs an SM is to hold (0: registers as the code wants them)
+template <class SH, int PER_SM>
+__global__ void __launch_bounds__(32 * SH::NB, PER_SM) forward_block_kernel(const KParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int s_item;
     float *sm = reinterpret_cast<float *>(smem_raw);

@@ -75,17 +75,16 @@ __device__ void bwd_rec_stripe_b(const KParams &P, int p, int si, const SmemB &L
         // ---- halo column t-63 (row i0+64) in shared memory before the step barrier;
         // a failed wait is flagged in misc[k & 1], read by every warp after the barrier
         const int jh = t - (ROWS - 1);
-        if (tid == 0 && has_below && jh >= 0 && jh <= Ly) {
+        if (q == 0 && has_below && jh >= 0 && jh <= Ly) {
             if (fetched > jh) {
-                if (!wait_geq(prog_below, Ly + 1 - jh, P.spin_limit)) {
-                    misc[k & 1] = 1;
+                int ok = 1;
+                if (lane == 0) ok = wait_geq(prog_below, Ly + 1 - jh, P.spin_limit) ? 1 : 0;
+                ok = __shfl_sync(0xffffffffu, ok, 0);
+                if (!ok) {
+                    if (lane == 0) misc[k & 1] = 1;
                 } else {
-                    const int sl = jh % 3;
-                    for (int i = 0; i < NS / 4; ++i)
-                        cp_async16(halo + sl * NS + 4 * i, edge_below + (int64_t)jh * NS + 4 * i);
-                    for (int i = 0; i < NBP / 4; ++i)
-                        cp_async16(haloE + sl * NBP + 4 * i, edgeE_below + (int64_t)jh * NBP + 4 * i);
-                    cp_commit();
+                    load_edge_warp(halo + (jh % 3) * NS, haloE + (jh % 3) * NBP, edge_below + (int64_t)jh * NS,
+                                   edgeE_below + (int64_t)jh * NBP, NS, NBP, lane);
                     fetched = jh;
                 }
             }
@@ -94,26 +93,27 @@ __device__ void bwd_rec_stripe_b(const KParams &P, int p, int si, const SmemB &L
         bar_sync(BAR_STEP, NB * 32);
         if (misc[k & 1]) { aborted = true; break; }
         // ---- top row of step t+1 -> edge row for the stripe above
-        if (tid == 0 && has_above && t + 1 <= T_last) {
+        if (q == 0 && has_above && t + 1 <= T_last) {
             const int jt = t + 1;
             if (jt <= Ly) {
-                copy_edge_cell(ring + ((t + 1) % 3) * ROWS * SPR, ringE + ((t + 1) % 3) * ROWS * NBP,
-                               edge_mine + (int64_t)jt * NS, edgeE_mine + (int64_t)jt * NBP, NS, NBP);
-                if ((jt % PUBB) == 0) st_release(prog_mine, Ly + 1 - jt);
+                store_edge_warp(ring + ((t + 1) % 3) * ROWS * SPR, ringE + ((t + 1) % 3) * ROWS * NBP,
+                                edge_mine + (int64_t)jt * NS, edgeE_mine + (int64_t)jt * NBP, NS, NBP, lane);
+                if ((jt % PUBB) == 0) {
+                    __threadfence();
+                    __syncwarp();
+                    if (lane == 0) st_release(prog_mine, Ly + 1 - jt);
+                }
             }
         }
         // ---- prefetch halo column jh-1 for the next step
-        if (tid == 0 && has_below && jh - 1 >= 0 && jh - 1 <= Ly) {
-            if (fetched == jh && pv >= Ly + 1 - (jh - 1)) {
-                const int sl = (jh - 1) % 3;
-                for (int i = 0; i < NS / 4; ++i)
-                    cp_async16(halo + sl * NS + 4 * i, edge_below + (int64_t)(jh - 1) * NS + 4 * i);
-                for (int i = 0; i < NBP / 4; ++i)
-                    cp_async16(haloE + sl * NBP + 4 * i, edgeE_below + (int64_t)(jh - 1) * NBP + 4 * i);
-                cp_commit();
+        if (q == 0 && has_below && jh - 1 >= 0 && jh - 1 <= Ly) {
+            const int sl = (jh - 1) % 3;
+            if (__shfl_sync(0xffffffffu, (fetched == jh && pv >= Ly + 1 - (jh - 1)) ? 1 : 0, 0)) {
+                load_edge_warp(halo + sl * NS, haloE + sl * NBP, edge_below + (int64_t)(jh - 1) * NS,
+                               edgeE_below + (int64_t)(jh - 1) * NBP, NS, NBP, lane);
                 fetched = jh - 1;
             }
-            if (pv < Ly + 3 - jh) pv = ld_acquire(prog_below);   // only when the next prefetch needs more
+            if (lane == 0 && pv < Ly + 3 - jh) pv = ld_acquire(prog_below);   // only when the next prefetch needs more
         }
         if (tid == 0) misc[(k + 1) & 1] = 0;   // every warp read it two barriers ago
         // ---- successor vectors of both cells (the zero vector when one does not exist)
@@ -167,7 +167,8 @@ __device__ void bwd_rec_stripe_b(const KParams &P, int p, int si, const SmemB &L
                 Eref[c] = max(Eref[c], Ed[c][d]);
             }
         }
-        float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f, g0 = 0.f, g1 = 0.f, g2 = 0.f, g3 = 0.f;
+        const float2 z2 = make_float2(0.f, 0.f);
+        float2 al = z2, ah = z2, gl = z2, gh = z2;
 #pragma unroll
         for (int d = 0; d < NB; ++d) {
             const int dt = P.quad_type[d];
@@ -188,11 +189,13 @@ __device__ void bwd_rec_stripe_b(const KParams &P, int p, int si, const SmemB &L
                     const float4 cv = chi4q[kk * (NS / 4)];
                     c0 = cv.x; c1 = cv.y; c2 = cv.z; c3 = cv.w;
                 }
-                a0 = fmaf(xs[ii], c0, a0); a1 = fmaf(xs[ii], c1, a1); a2 = fmaf(xs[ii], c2, a2); a3 = fmaf(xs[ii], c3, a3);
-                g0 = fmaf(yv[ii], c0, g0); g1 = fmaf(yv[ii], c1, g1); g2 = fmaf(yv[ii], c2, g2); g3 = fmaf(yv[ii], c3, g3);
+                const float2 kl = make_float2(c0, c1), kh = make_float2(c2, c3);
+                const float2 x2 = make_float2(xs[ii], xs[ii]), y2 = make_float2(yv[ii], yv[ii]);
+                al = __ffma2_rn(x2, kl, al); ah = __ffma2_rn(x2, kh, ah);
+                gl = __ffma2_rn(y2, kl, gl); gh = __ffma2_rn(y2, kh, gh);
             }
         }
-        const float4 accv[R] = {make_float4(a0, a1, a2, a3), make_float4(g0, g1, g2, g3)};
+        const float4 accv[R] = {make_float4(al.x, al.y, ah.x, ah.y), make_float4(gl.x, gl.y, gh.x, gh.y)};
 #pragma unroll
         for (int c = 0; c < R; ++c) {
             const int rho = lane + 32 * c;
@@ -228,8 +231,8 @@ __device__ void bwd_rec_stripe_b(const KParams &P, int p, int si, const SmemB &L
         }
     }
     bar_sync(BAR_STEP, NB * 32);   // step 0's ring is complete
+    if (q == 0) cp_wait0();
     if (tid == 0) {
-        cp_wait0();
         if (has_above) {
             if (!aborted)
                 copy_edge_cell(ring, ringE, edge_mine, edgeE_mine, NS, NBP);   // column 0 (step 0)
@@ -249,8 +252,8 @@ __device__ void bwd_rec_stripe_b(const KParams &P, int p, int si, const SmemB &L
 // only for a stripe of its own direction popped before it.
 constexpr int BWD_ITEM = 1 << 30;
 
-template <class SH>
-__global__ void __launch_bounds__(32 * SH::NB) fwdbwd_block_kernel(const KParams P) {
+template <class SH, int PER_SM>
+__global__ void __launch_bounds__(32 * SH::NB, PER_SM) fwdbwd_block_kernel(const KParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int s_item;
     float *sm = reinterpret_cast<float *>(smem_raw);

@@ -2230,8 +2230,15 @@ int launch_block(phmm_plan *plan, KParams &K, int n_items, int max_ly, int kind,
         threads = blk::CNT_THREADS;
     } else {
         bytes = blk::make_smem_b(SH::NS, SH::NB, 1, K.G, max_ly, kind == 1).bytes;
-        kern = kind == 0 ? blk::forward_block_kernel<SH>
-                         : (kind == 1 ? blk::backward_block_kernel<SH> : blk::fwdbwd_block_kernel<SH>);
+        kern = kind == 0 ? blk::forward_block_kernel<SH, 0>
+                         : (kind == 1 ? blk::backward_block_kernel<SH> : blk::fwdbwd_block_kernel<SH, 0>);
+        // 44 slots, more stripes than SMs: two CTAs an SM at 80 registers (one at 129 issues in 60 % of
+        // the cycles at best; 32 pairs of 200-1500: 16.0 ms, two 15.1).  A stripe alone is faster
+        // with its registers (one pair of 511 x 600, forward: 2.53 ms against 2.60).
+        if constexpr (!SH::CHI_REG) {
+            if (n_items > plan->sm_count && kind == 0) kern = blk::forward_block_kernel<SH, 2>;
+            if (n_items > plan->sm_count && kind == 4) kern = blk::fwdbwd_block_kernel<SH, 2>;
+        }
         threads = 32 * (SH::NB + (kind == 1 ? blk::NCW : 0));
     }
     CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
