@@ -999,23 +999,24 @@ __device__ void count_stripe_wd(const KParams &P, int p, int si, int sp, const S
             const int tile = tid + a * CT;
             if (tile >= ntile) continue;
             const int bs = tile / NQd, bk = tile % NQd;
-            float pz[16];
+            float2 pz[8];   // pairs of destinations: one issue for two multiply-adds
 #pragma unroll
-            for (int u = 0; u < 16; ++u) pz[u] = 0.f;
+            for (int u = 0; u < 8; ++u) pz[u] = make_float2(0.f, 0.f);
 #pragma unroll 4
             for (int rr = 0; rr < RW; ++rr) {
                 const float4 fv4 = *reinterpret_cast<const float4 *>(fst + rr * FW + 4 * bs);
                 const float4 uv4 = *reinterpret_cast<const float4 *>(ust + rr * UW + 4 * bk);
                 const float fa[4] = {fv4.x, fv4.y, fv4.z, fv4.w};
-                const float ua[4] = {uv4.x, uv4.y, uv4.z, uv4.w};
+                const float2 ul = make_float2(uv4.x, uv4.y), uh = make_float2(uv4.z, uv4.w);
 #pragma unroll
-                for (int x = 0; x < 4; ++x)
-#pragma unroll
-                    for (int y = 0; y < 4; ++y) pz[4 * x + y] = fmaf(fa[x], ua[y], pz[4 * x + y]);
+                for (int x = 0; x < 4; ++x) {
+                    pz[2 * x] = __ffma2_rn(make_float2(fa[x], fa[x]), ul, pz[2 * x]);
+                    pz[2 * x + 1] = __ffma2_rn(make_float2(fa[x], fa[x]), uh, pz[2 * x + 1]);
+                }
             }
 #pragma unroll
             for (int u = 0; u < 16; ++u) {
-                const float y = pz[u] - ccomp[a][u];
+                const float y = (u & 1 ? pz[u / 2].y : pz[u / 2].x) - ccomp[a][u];
                 const float tt = csum[a][u] + y;
                 ccomp[a][u] = (tt - csum[a][u]) - y;
                 csum[a][u] = tt;

@@ -388,7 +388,12 @@ __device__ void fwd_stripe_wn(const KParams &P, int p, int si, const SmemWn &L, 
 #pragma unroll
                     for (int i = 0; i < 4; ++i)
 #pragma unroll
-                        for (int u = 0; u < 4; ++u) acc[i][u] = fmaf(pa[i], ca[u], acc[i][u]);
+                        for (int u = 0; u < 4; u += 2) {   // one issue for two multiply-adds
+                            const float2 o = __ffma2_rn(make_float2(pa[i], pa[i]), make_float2(ca[u], ca[u + 1]),
+                                                        make_float2(acc[i][u], acc[i][u + 1]));
+                            acc[i][u] = o.x;
+                            acc[i][u + 1] = o.y;
+                        }
                 }
             }
             // the start state (non-zero only at the origin) for the cells next to it
@@ -741,7 +746,12 @@ __device__ void bwd_rec_stripe_wn(const KParams &P, int p, int si, const SmemWn 
 #pragma unroll
                     for (int i = 0; i < 4; ++i)
 #pragma unroll
-                        for (int u = 0; u < 4; ++u) acc[i][u] = fmaf(wa[i], ca[u], acc[i][u]);
+                        for (int u = 0; u < 4; u += 2) {   // one issue for two multiply-adds
+                            const float2 o = __ffma2_rn(make_float2(wa[i], wa[i]), make_float2(ca[u], ca[u + 1]),
+                                                        make_float2(acc[i][u], acc[i][u + 1]));
+                            acc[i][u] = o.x;
+                            acc[i][u + 1] = o.y;
+                        }
                 }
             }
             float bv[4][4], mxr[4];
