@@ -778,6 +778,7 @@ __global__ void __launch_bounds__(512) fwdbwd_wide_kernel(const KParams P) {
 // character, float64 reductions at the end of the stripe).
 constexpr int CT = 512;          // count CTA
 constexpr int SPL = 2;           // source-slot halves per stripe
+constexpr int CSTEPS = 96;       // least steps of a count item that is a run of a stripe's steps
 constexpr int CTPT = 2;          // outer-product tiles per thread (ceil(NQ/2) * NQd <= CT * CTPT)
 
 struct SmemWc {
@@ -800,7 +801,8 @@ __host__ __device__ inline SmemWc make_smem_wc(int NS, int KS, int wM, int wI, i
     return L;
 }
 
-__device__ void count_stripe_wd(const KParams &P, int p, int si, int sp, const SmemWc &L, float *sm) {
+// part: which of the P.count_split runs of steps
+__device__ void count_stripe_wd(const KParams &P, int p, int si, int sp, int part, const SmemWc &L, float *sm) {
     const int NS = P.NS, KS = P.kend[2], NQd = KS / 4, NQ = NS / 4, N = P.N, G = P.G;
     const int SQ = (NQ + SPL - 1) / SPL;
     const int sq0 = sp * SQ, sq1 = min(NQ, sq0 + SQ), nsq = sq1 - sq0;
@@ -818,7 +820,9 @@ __device__ void count_stripe_wd(const KParams &P, int p, int si, int sp, const S
     // backward edge row, whose records hold w = e b (the emission already applied)
     const float *bedge_below = P.bedge + (m.edge_base + (int64_t)(si + 1) * (Ly + 1)) * ES;
     const int T_last = (nrows - 1) + Ly;
-    if (nsq <= 0) return;
+    const int len = max(CSTEPS, (T_last + P.count_split) / P.count_split);
+    const int t_hi = T_last - part * len, t_lo = max(0, t_hi - len + 1);
+    if (nsq <= 0 || t_hi < 0) return;
     if (P.count_wait) {   // the wavefronts may still run: wait for the stripes read here
         __shared__ int s_ok;
         if (tid == 0) {
@@ -880,7 +884,7 @@ __device__ void count_stripe_wd(const KParams &P, int p, int si, int sp, const S
     float4 sv[KQ], fv[FQ], bo[KQ];
     auto issue = [&](int t) {
         const int j = t - c;
-        const bool valid = t >= 0 && c < nrows && j >= 0 && j <= Ly;
+        const bool valid = t >= t_lo && c < nrows && j >= 0 && j <= Ly;
         const int64_t cell = latc + (int64_t)t * RW + c;
         Ef = EXP_NONE; Eb = EXP_NONE;
 #pragma unroll
@@ -921,8 +925,8 @@ __device__ void count_stripe_wd(const KParams &P, int p, int si, int sp, const S
             }
         }
     };
-    issue(T_last);
-    for (int t = T_last; t >= 0; --t) {
+    issue(t_hi);
+    for (int t = t_hi; t >= t_lo; --t) {
         // ================= phase A
         {
             const int j = t - c;
@@ -1076,8 +1080,8 @@ __global__ void __launch_bounds__(CT, 1) count_wide_kernel(const KParams P) {
         __syncthreads();
         const int it = s_item;
         if (it >= P.n_items) break;
-        const int2 w = P.items[it];
-        count_stripe_wd(P, w.x, w.y >> 4, w.y & 15, L, sm);
+        const int2 w = P.items[it / P.count_split];
+        count_stripe_wd(P, w.x, w.y >> 4, w.y & 15, it % P.count_split, L, sm);
     }
 }
 

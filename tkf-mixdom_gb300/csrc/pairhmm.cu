@@ -114,6 +114,7 @@ struct KParams {
     // stripe (global stripe index) in the current group's scratch, or null
     // for the full-lattice layout (PairMeta::lat_base)
     const int64_t *stripe_lat;
+    int count_split;     // wide count pass: runs of steps a stripe is counted in (1: whole)
     int recompute;                      // 1: stripes recomputed from complete edge rows (no waits, no
                                         // edge / progress / log-likelihood writes)
     int ckpt;                           // count pass: row 0 of the stripe below from its backward edge row
@@ -1485,6 +1486,7 @@ int run_wide(phmm_plan *plan, const phmm_batch *b, bool estep, double *ll, doubl
              double *cntI, double *cntD, int32_t *status, cudaStream_t stream, void *ws, size_t ws_bytes,
              size_t *ws_need) {
     KParams K = plan->base;
+    K.count_split = 1;
     const int P_ = b->n_pairs, N = K.N, G = K.G, NS = K.NS;
     const int KS = K.kend[2], NQd = KS / 4, NQ = NS / 4;
     const int ES = wide::ls_of(NS);
@@ -1784,9 +1786,15 @@ int run_wide(phmm_plan *plan, const phmm_batch *b, bool estep, double *ll, doubl
         if (plan->timing) CUDA_TRY(cudaEventRecord(plan->ev[4], stream));
         if (!ckpt) {
             K.items = (const int2 *)d_items + n_fb;
-            K.n_items = n_citems;
+            // few stripes: each half-stripe in runs of steps, so that the last ones to start do
+            // not leave the other SMs idle (4 pairs of 700-1100 at 162 states, 232 halves on 152
+            // SMs: 15.7 ms, in runs 11.5); a run costs a clearing and a flush of the counts, so no
+            // more than about six to an SM and none under CSTEPS
+            const int slots = plan->sm_count * occ;
+            K.count_split = std::max(1, std::min((6 * slots + n_citems - 1) / n_citems, (max_ly + rows) / wide::CSTEPS));
+            K.n_items = n_citems * K.count_split;
             K.counter = d_counters + 2;
-            wide::count_wide_kernel<<<std::min(n_citems, plan->sm_count * occ), wide::CT, bytes, stream>>>(K);
+            wide::count_wide_kernel<<<std::min(K.n_items, slots), wide::CT, bytes, stream>>>(K);
             CUDA_TRY(cudaGetLastError());
             plan->launches++;
         } else {
