@@ -155,6 +155,65 @@ struct QuadEmit {
     __device__ __forceinline__ float at(int i, int u, int y) const { return __ldg(tab + gb[u] + xo[i] + ym * y); }
 };
 
+// The rows' type sums and maxima meet in shared memory.  A warp's lanes are four quads
+// (lane bits 3, 4) of eight row groups, four rows a lane: quads that add to the same sums are
+// added in the warp first, each lane keeping a part of the rows, so a lane has one
+// row's atomics left instead of four rows' that three others collide with (a float
+// addition in shared memory is a compare-and-swap loop: 4 pairs of 700-1100 at 162 states,
+// both recursions, 20.1 ms; added in the warp first 16.8).
+struct QuadPeers {
+    bool lo, hi, s8, s16;   // lane bits 3, 4; the quads across them add to the same sums (as the whole warp's do)
+    __device__ void init(int lane, int key) {   // key < 0: an inactive quad
+        lo = lane & 8;
+        hi = lane & 16;
+        s16 = __all_sync(0xffffffffu, key >= 0 && key == __shfl_xor_sync(0xffffffffu, key, 16));
+        s8 = s16 && __all_sync(0xffffffffu, key == __shfl_xor_sync(0xffffffffu, key, 8));
+    }
+    // v[i][a]: value a of row i of this lane's four, to dst[a * stride + i]
+    template <int NV>
+    __device__ void add(const float (&v)[4][NV], float *dst, int stride) const {
+        if (!s16) {   // uniform over the warp
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int a = 0; a < NV; ++a)
+                    if (v[i][a] != 0.f) atomicAdd(dst + a * stride + i, v[i][a]);
+            return;
+        }
+        float w[2][NV];
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int a = 0; a < NV; ++a)
+                w[i][a] = (hi ? v[i + 2][a] : v[i][a]) + __shfl_xor_sync(0xffffffffu, hi ? v[i][a] : v[i + 2][a], 16);
+        dst += hi ? 2 : 0;
+        if (!s8) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int a = 0; a < NV; ++a)
+                    if (w[i][a] != 0.f) atomicAdd(dst + a * stride + i, w[i][a]);
+            return;
+        }
+        dst += lo ? 1 : 0;
+#pragma unroll
+        for (int a = 0; a < NV; ++a) {
+            const float x = (lo ? w[1][a] : w[0][a]) + __shfl_xor_sync(0xffffffffu, lo ? w[0][a] : w[1][a], 8);
+            if (x != 0.f) atomicAdd(dst + a * stride, x);
+        }
+    }
+    // maxima (positive float bits) of the four rows, over all quads
+    __device__ void max(const float (&m)[4], int *dst) const {
+        int w[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+            w[i] = ::max(__float_as_int(hi ? m[i + 2] : m[i]),
+                         __shfl_xor_sync(0xffffffffu, __float_as_int(hi ? m[i] : m[i + 2]), 16));
+        const int x = ::max(lo ? w[1] : w[0], __shfl_xor_sync(0xffffffffu, lo ? w[0] : w[1], 8));
+        if (x > 0) atomicMax(dst + (hi ? 2 : 0) + (lo ? 1 : 0), x);
+    }
+};
+
 // ---------------------------------------------------------------- forward
 __device__ void fwd_stripe_wn(const KParams &P, int p, int si, const SmemWn &L, float *sm, unsigned char *smb) {
     const int NS = P.NS, KS = P.kend[2], NQd = KS / 4;
@@ -234,6 +293,8 @@ __device__ void fwd_stripe_wn(const KParams &P, int p, int si, const SmemWn &L, 
         }
     }
     const float *iaq = sm + L.ia + (active ? qd : 0) * NIA;
+    QuadPeers peers;
+    peers.init(lane, active ? myU : -1);
     // halo column col of row i0-1: B slot (col - 1) % 3 index 0, E / MX slot
     // (col - 1) & 3, and its type sums in G slot (col - 1) & 3 index 0 (warp 0)
     // The halo column is loaded into registers one step before it is staged
@@ -328,6 +389,7 @@ __device__ void fwd_stripe_wn(const KParams &P, int p, int si, const SmemWn &L, 
                 }
             }
         }
+        float gsum[4][1] = {{0.f}, {0.f}, {0.f}, {0.f}}, mxr[4] = {0.f, 0.f, 0.f, 0.f};
         if (active) {
             int Eo[4];
             float sc[4];
@@ -405,13 +467,11 @@ __device__ void fwd_stripe_wn(const KParams &P, int p, int si, const SmemWn &L, 
 #pragma unroll
                     for (int u = 0; u < 4; ++u) acc[i][u] = fmaf(pa[i], sm[L.c0 + 4 * qd + u], acc[i][u]);
             }
-            float mxr[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int r = r0 + i, j = t - r;
                 const int yj = valid[i] ? ys[j] : 0;
                 const bool origin = valid[i] && i0 + r == 0 && j == 0;
-                mxr[i] = 0.f;
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     float v = 0.f;
@@ -435,10 +495,8 @@ __device__ void fwd_stripe_wn(const KParams &P, int p, int si, const SmemWn &L, 
                 const int r = r0 + i, row = i0 + r, j = t - r;
                 const bool origin = valid[i] && row == 0 && j == 0;
                 if (qd == 0) E[(t & 3) * BW + r + 1] = origin ? 0 : Eo[i];
-                if (mxr[i] > 0.f) atomicMax(MX + (t & 3) * BW + r + 1, __float_as_int(mxr[i]));
                 // my quad's share of the new cell's type sum
-                const float g = fmaf(exr[3], acc[i][3], fmaf(exr[2], acc[i][2], fmaf(exr[1], acc[i][1], exr[0] * acc[i][0])));
-                if (g != 0.f) atomicAdd(GB + (t & 3) * GS + myU * BW + r + 1, g);
+                gsum[i][0] = fmaf(exr[3], acc[i][3], fmaf(exr[2], acc[i][2], fmaf(exr[1], acc[i][1], exr[0] * acc[i][0])));
                 if (valid[i] && P.lat) {
                     const int64_t cell = latc + (int64_t)t * RW + r;
                     float *rec = P.lat + cell * ES;
@@ -462,6 +520,8 @@ __device__ void fwd_stripe_wn(const KParams &P, int p, int si, const SmemWn &L, 
                 atomicMax(MX + 0 * BW + 1, __float_as_int(1.f));
             }
         }
+        peers.max(mxr, MX + (t & 3) * BW + r0 + 1);
+        peers.add<1>(gsum, GB + (t & 3) * GS + myU * BW + r0 + 1, BW);
         if (warp == 0 && t + 1 <= T_last) {   // column t+1 (loaded last step) staged; t+2 loaded
             stage_halo(t + 1);
             if (t + 2 <= T_last && !load_halo(t + 2) && lane == 0) misc[(k + 1) & 1] = 1;
@@ -586,6 +646,8 @@ __device__ void bwd_rec_stripe_wn(const KParams &P, int p, int si, const SmemWn 
         }
     }
     const float *iaq = sm + L.ia + (active ? qs : 0) * NIA;
+    QuadPeers peers;
+    peers.init(lane, active ? myT : -1);
     int tqr[3];   // the partner quads' destination types
 #pragma unroll
     for (int j = 0; j < 3; ++j) tqr[j] = pqr[j] >= 0 ? P.quad_type[pqr[j]] : T_NONE;
@@ -681,6 +743,9 @@ __device__ void bwd_rec_stripe_wn(const KParams &P, int p, int si, const SmemWn 
             if (idx % BW != RW + 3) PR[((t - 1) & 3) * PS + idx] = 0.f;
         }
         if (warp == (nt > 32 ? 1 : 0)) publish_top(t + 1);
+        float psum[4][3], mxr[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) psum[i][0] = psum[i][1] = psum[i][2] = mxr[i] = 0.f;
         if (active) {
             int Eo[4], EsM[4], EsI[4], EsD[4];
             bool valid[4], term[4];
@@ -754,12 +819,11 @@ __device__ void bwd_rec_stripe_wn(const KParams &P, int p, int si, const SmemWn 
                         }
                 }
             }
-            float bv[4][4], mxr[4];
+            float bv[4][4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int r = r0 + i, j = t - r;
                 const int yj = valid[i] ? ys[j] : 0;
-                mxr[i] = 0.f;
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     float b = 0.f;
@@ -786,12 +850,9 @@ __device__ void bwd_rec_stripe_wn(const KParams &P, int p, int si, const SmemWn 
                 }
                 // my quad's share of the new cell's P sums (my quad as destinations of type myT)
 #pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    const float pa = fmaf(cinr[a][3], wv[3], fmaf(cinr[a][2], wv[2], fmaf(cinr[a][1], wv[1], cinr[a][0] * wv[0])));
-                    if (pa != 0.f) atomicAdd(PR + (t & 3) * PS + (3 * myT + a) * BW + r + 3, pa);
-                }
+                for (int a = 0; a < 3; ++a)
+                    psum[i][a] = fmaf(cinr[a][3], wv[3], fmaf(cinr[a][2], wv[2], fmaf(cinr[a][1], wv[1], cinr[a][0] * wv[0])));
                 if (qs == 0) E[(t & 3) * BW + r] = valid[i] ? Eo[i] : EXP_NONE;
-                if (mxr[i] > 0.f) atomicMax(MX + (t & 3) * BW + r, __float_as_int(mxr[i]));
                 if (valid[i] && P.blat) {
                     const int64_t cell = latc + (int64_t)t * RW + r;
                     float *rec = P.blat + cell * ES;
@@ -800,6 +861,8 @@ __device__ void bwd_rec_stripe_wn(const KParams &P, int p, int si, const SmemWn 
                 }
             }
         }
+        peers.max(mxr, MX + (t & 3) * BW + r0);
+        peers.add<3>(psum, PR + (t & 3) * PS + 3 * myT * BW + r0 + 3, BW);
         if (warp == 0) {   // column t - RW (loaded last step) staged; the next one loaded
             stage_halo(t - RW);
             if (!load_halo(t - RW - 1) && lane == 0) misc[(k + 1) & 1] = 1;
