@@ -160,7 +160,8 @@ struct QuadEmit {
 // added in the warp first, each lane keeping a part of the rows, so a lane has one
 // row's atomics left instead of four rows' that three others collide with (a float
 // addition in shared memory is a compare-and-swap loop: 4 pairs of 700-1100 at 162 states,
-// both recursions, 20.1 ms; added in the warp first 16.8).
+// both recursions, 20.1 ms; added in the warp first 16.8, and with the boundary rows moved by two
+// warps that have no quads 14.9).
 struct QuadPeers {
     bool lo, hi, s8, s16;   // lane bits 3, 4; the quads across them add to the same sums (as the whole warp's do)
     __device__ void init(int lane, int key) {   // key < 0: an inactive quad
@@ -220,6 +221,7 @@ __device__ void fwd_stripe_wn(const KParams &P, int p, int si, const SmemWn &L, 
     const PairMeta m = P.meta[p];
     const int Lx = m.Lx, Ly = m.Ly;
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
+    const int halo_warp = nt / 32 - 1, pub_warp = nt / 32 - 2;   // no quads of their own
     const int rg = lane & 7, qd = 4 * warp + (lane >> 3);
     const bool active = qd < NQd;
     const int r0 = 4 * rg;
@@ -296,14 +298,14 @@ __device__ void fwd_stripe_wn(const KParams &P, int p, int si, const SmemWn &L, 
     QuadPeers peers;
     peers.init(lane, active ? myU : -1);
     // halo column col of row i0-1: B slot (col - 1) % 3 index 0, E / MX slot
-    // (col - 1) & 3, and its type sums in G slot (col - 1) & 3 index 0 (warp 0)
+    // (col - 1) & 3, and its type sums in G slot (col - 1) & 3 index 0 (the halo warp)
     // The halo column is loaded into registers one step before it is staged
-    // (its L2 latency then overlaps a whole step instead of holding warp 0
+    // (its L2 latency then overlaps a whole step instead of holding its warp
     // -- and with it the step's barrier -- at the end of each step).
     constexpr int HQ = (WMAXS + 31) / 32;
     float hv[HQ];
     int hE = EXP_NONE, hMX = 0;
-    auto load_halo = [&](int col) -> bool {   // warp 0
+    auto load_halo = [&](int col) -> bool {   // halo warp
         if (!has_above || col > Ly) return true;
         int ok = 1;
         if (lane == 0) ok = wait_geq(prog_above, col + 1, P.spin_limit) ? 1 : 0;
@@ -321,7 +323,7 @@ __device__ void fwd_stripe_wn(const KParams &P, int p, int si, const SmemWn &L, 
         }
         return true;
     };
-    auto stage_halo = [&](int col) {   // warp 0: the loaded column into B, E / MX and its type sums
+    auto stage_halo = [&](int col) {   // halo warp: the loaded column into B, E / MX and its type sums
         if (!has_above || col > Ly) return;
         const int bs = (col + 2) % 3, es = (col + 3) & 3;
         float g[3] = {0.f, 0.f, 0.f};
@@ -349,7 +351,7 @@ __device__ void fwd_stripe_wn(const KParams &P, int p, int si, const SmemWn &L, 
         }
     };
     __syncthreads();
-    if (warp == 0) {
+    if (warp == halo_warp) {
         bool ok = load_halo(0);
         if (ok) stage_halo(0);
         if (ok) ok = load_halo(1);
@@ -365,14 +367,14 @@ __device__ void fwd_stripe_wn(const KParams &P, int p, int si, const SmemWn &L, 
         for (int r = tid; r < RW; r += nt) MX[((t + 1) & 3) * BW + r + 1] = 0;
         // the G slot of step t+1 starts at zero (last read at step t-1, as an M-predecessor)
         for (int idx = tid; idx < GS; idx += nt) {
-            if (idx % BW != 0) GB[((t + 1) & 3) * GS + idx] = 0.f;   // index 0: the halo row, written by warp 0
+            if (idx % BW != 0) GB[((t + 1) & 3) * GS + idx] = 0.f;   // index 0: the halo row, written by the halo warp
         }
         if (si == 0 && tid == 0 && P.s_slot >= KS) {
             if (t == 2) A[(0 * NS + P.s_slot) * RW + 0] = 0.f;
             if (t == 3) B[(0 * NS + P.s_slot) * BW + 1] = 0.f;
         }
-        // ---- bottom row of step t-1 -> edge row for the stripe below (warp 1)
-        if (warp == (nt > 32 ? 1 : 0) && has_below && t >= 1) {
+        // ---- bottom row of step t-1 -> edge row for the stripe below (the publishing warp)
+        if (warp == pub_warp && has_below && t >= 1) {
             const int jb = t - 1 - (RW - 1);
             if (jb >= 0 && jb <= Ly) {
                 const int sl = (t - 1) % 3;
@@ -520,9 +522,11 @@ __device__ void fwd_stripe_wn(const KParams &P, int p, int si, const SmemWn &L, 
                 atomicMax(MX + 0 * BW + 1, __float_as_int(1.f));
             }
         }
-        peers.max(mxr, MX + (t & 3) * BW + r0 + 1);
-        peers.add<1>(gsum, GB + (t & 3) * GS + myU * BW + r0 + 1, BW);
-        if (warp == 0 && t + 1 <= T_last) {   // column t+1 (loaded last step) staged; t+2 loaded
+        if (warp < pub_warp) {
+            peers.max(mxr, MX + (t & 3) * BW + r0 + 1);
+            peers.add<1>(gsum, GB + (t & 3) * GS + myU * BW + r0 + 1, BW);
+        }
+        if (warp == halo_warp && t + 1 <= T_last) {   // column t+1 (loaded last step) staged; t+2 loaded
             stage_halo(t + 1);
             if (t + 2 <= T_last && !load_halo(t + 2) && lane == 0) misc[(k + 1) & 1] = 1;
         }
@@ -531,7 +535,7 @@ __device__ void fwd_stripe_wn(const KParams &P, int p, int si, const SmemWn &L, 
     if (!aborted && has_below) {
         const int t = T_last + 1;
         const int jb = t - 1 - (RW - 1);
-        if (warp == (nt > 32 ? 1 : 0) && jb >= 0 && jb <= Ly) {
+        if (warp == pub_warp && jb >= 0 && jb <= Ly) {
             const int sl = (t - 1) % 3;
             float *dst = edge_mine + (int64_t)jb * ES;
             for (int s = lane; s < NS; s += 32) dst[s] = B[(sl * NS + s) * BW + RW];
@@ -577,6 +581,7 @@ __device__ void bwd_rec_stripe_wn(const KParams &P, int p, int si, const SmemWn 
     const PairMeta m = P.meta[p];
     const int Lx = m.Lx, Ly = m.Ly;
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
+    const int halo_warp = nt / 32 - 1, pub_warp = nt / 32 - 2;   // no quads of their own
     const int rg = lane & 7, qs = 4 * warp + (lane >> 3);   // output (source) quad
     const bool active = qs < NQd;
     const int r0 = 4 * rg;
@@ -656,7 +661,7 @@ __device__ void bwd_rec_stripe_wn(const KParams &P, int p, int si, const SmemWn 
     constexpr int HQ = (WMAXS + 31) / 32;
     float hv[HQ];
     int hE = EXP_NONE, hMX = 0;
-    auto load_halo = [&](int col) -> bool {   // warp 0 (loaded a step before staged, as in the forward)
+    auto load_halo = [&](int col) -> bool {   // halo warp (loaded a step before staged, as in the forward)
         if (!has_below || col < 0 || col > Ly) return true;
         int ok = 1;
         if (lane == 0) ok = wait_geq(prog_below, Ly + 1 - col, P.spin_limit) ? 1 : 0;
@@ -724,7 +729,7 @@ __device__ void bwd_rec_stripe_wn(const KParams &P, int p, int si, const SmemWn 
         }
     };
     __syncthreads();
-    if (warp == 0) {
+    if (warp == halo_warp) {
         bool ok = load_halo(T_last - (RW - 1));
         if (ok) stage_halo(T_last - (RW - 1));
         if (ok) ok = load_halo(T_last - RW);
@@ -738,11 +743,11 @@ __device__ void bwd_rec_stripe_wn(const KParams &P, int p, int si, const SmemWn 
         if (tid == 0) misc[(k + 1) & 1] = 0;
         for (int r = tid; r < RW; r += nt) MX[((t - 1) & 3) * BW + r] = 0;
         // the P slot of step t-1 starts at zero (last read at step t+1, as an
-        // M-successor); its halo index RW + 3 is written by warp 0
+        // M-successor); its halo index RW + 3 is written by the halo warp
         for (int idx = tid; idx < PS; idx += nt) {
             if (idx % BW != RW + 3) PR[((t - 1) & 3) * PS + idx] = 0.f;
         }
-        if (warp == (nt > 32 ? 1 : 0)) publish_top(t + 1);
+        if (warp == pub_warp) publish_top(t + 1);
         float psum[4][3], mxr[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) psum[i][0] = psum[i][1] = psum[i][2] = mxr[i] = 0.f;
@@ -861,15 +866,17 @@ __device__ void bwd_rec_stripe_wn(const KParams &P, int p, int si, const SmemWn 
                 }
             }
         }
-        peers.max(mxr, MX + (t & 3) * BW + r0);
-        peers.add<3>(psum, PR + (t & 3) * PS + 3 * myT * BW + r0 + 3, BW);
-        if (warp == 0) {   // column t - RW (loaded last step) staged; the next one loaded
+        if (warp < pub_warp) {
+            peers.max(mxr, MX + (t & 3) * BW + r0);
+            peers.add<3>(psum, PR + (t & 3) * PS + 3 * myT * BW + r0 + 3, BW);
+        }
+        if (warp == halo_warp) {   // column t - RW (loaded last step) staged; the next one loaded
             stage_halo(t - RW);
             if (!load_halo(t - RW - 1) && lane == 0) misc[(k + 1) & 1] = 1;
         }
     }
     __syncthreads();
-    if (!aborted && warp == (nt > 32 ? 1 : 0)) publish_top(0);
+    if (!aborted && warp == pub_warp) publish_top(0);
     __syncthreads();
     if (tid == 0) {
         if (has_above) { __threadfence(); st_release(prog_mine, Ly + 1); }
@@ -883,7 +890,7 @@ __device__ void bwd_rec_stripe_wn(const KParams &P, int p, int si, const SmemWn 
 // Persistent CTAs over interleaved forward and backward stripe items (E-step),
 // or forward items only.
 template <bool FWD_ONLY>
-__global__ void __launch_bounds__(384) wide_nest_kernel(const KParams P) {   // 32 x 12 warps at most (48 quads)
+__global__ void __launch_bounds__(384) wide_nest_kernel(const KParams P) {   // four quads a warp (at most 40), halo, publishing
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int s_item;
     float *sm = reinterpret_cast<float *>(smem_raw);

@@ -1746,7 +1746,7 @@ int run_wide(phmm_plan *plan, const phmm_batch *b, bool estep, double *ll, doubl
         K.items = (const int2 *)d_items;
         K.n_items = n_fb;
         K.counter = d_counters;
-        const int threads = 32 * ((NQd + 3) / 4);
+        int threads = 32 * ((NQd + 3) / 4);
         int bytes = std::max(wide::make_smem_wd(NS, KS, max_ly, false).bytes,
                              estep ? wide::make_smem_wd(NS, KS, max_ly, true).bytes : 0);
         auto kern = estep ? fb_kernel : f_kernel;
@@ -1756,6 +1756,7 @@ int run_wide(phmm_plan *plan, const phmm_batch *b, bool estep, double *ll, doubl
             K.nest_K = b->nest_dom;
             K.nest_F = b->nest_frag;
             kern = estep ? wide::wide_nest_kernel<false> : wide::wide_nest_kernel<true>;
+            threads += 64;   // the boundary rows in and out by warps of their own
             bytes = std::max(wide::make_smem_wn(NS, KS, max_ly, false).bytes,
                              estep ? wide::make_smem_wn(NS, KS, max_ly, true).bytes : 0);
         }
