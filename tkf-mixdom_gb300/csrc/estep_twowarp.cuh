@@ -1589,7 +1589,7 @@ __device__ void count_chunk_teams(const KParams &P, int p, int si, int ch, const
 
     int n_prev = 0;
     for (int tt = t_hi; tt >= t_lo; tt -= T) {
-        const int n = min(T, tt - t_lo + 1), t = tt - team;   // steps of this round
+        const int n = min(T, tt - t_lo + 1), t = tt - team;   // steps of the round
         if (team < n) {
             const int jc = t - r;
             const bool valid = r < nrows && jc >= 0 && jc <= Ly;

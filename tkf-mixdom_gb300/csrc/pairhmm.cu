@@ -1785,14 +1785,15 @@ int run_wide(phmm_plan *plan, const phmm_batch *b, bool estep, double *ll, doubl
         CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, wide::count_wide_kernel, wide::CT, bytes));
         if (occ < 1) return fail(PHMM_E_ARG, "wide count kernel does not fit on an SM (shared memory)");
         if (plan->timing) CUDA_TRY(cudaEventRecord(plan->ev[4], stream));
+        // few stripes: each half-stripe in runs of steps, so that the last ones to start do
+        // not leave the other SMs idle (4 pairs of 700-1100 at 162 states, 232 halves on 152
+        // SMs: 15.7 ms, in runs 11.5); a run costs a clearing and a flush of the counts, so no
+        // more than about six to an SM and none under CSTEPS.  A checkpointed pass counts in the
+        // same runs: the emission counts of a run are float32 sums, so the runs set their rounding.
+        const int slots = plan->sm_count * occ;
+        K.count_split = std::max(1, std::min((6 * slots + n_citems - 1) / n_citems, (max_ly + rows) / wide::CSTEPS));
         if (!ckpt) {
             K.items = (const int2 *)d_items + n_fb;
-            // few stripes: each half-stripe in runs of steps, so that the last ones to start do
-            // not leave the other SMs idle (4 pairs of 700-1100 at 162 states, 232 halves on 152
-            // SMs: 15.7 ms, in runs 11.5); a run costs a clearing and a flush of the counts, so no
-            // more than about six to an SM and none under CSTEPS
-            const int slots = plan->sm_count * occ;
-            K.count_split = std::max(1, std::min((6 * slots + n_citems - 1) / n_citems, (max_ly + rows) / wide::CSTEPS));
             K.n_items = n_citems * K.count_split;
             K.counter = d_counters + 2;
             wide::count_wide_kernel<<<std::min(K.n_items, slots), wide::CT, bytes, stream>>>(K);
@@ -1823,9 +1824,9 @@ int run_wide(phmm_plan *plan, const phmm_batch *b, bool estep, double *ll, doubl
                 K.recompute = 0;
                 K.ckpt = 1;
                 K.items = (const int2 *)d_items + g.c_off;
-                K.n_items = (int)g.n_c;
+                K.n_items = (int)g.n_c * K.count_split;
                 K.counter = d_counters + 1;
-                wide::count_wide_kernel<<<std::min((int)g.n_c, plan->sm_count * occ), wide::CT, bytes, stream>>>(K);
+                wide::count_wide_kernel<<<std::min(K.n_items, slots), wide::CT, bytes, stream>>>(K);
                 CUDA_TRY(cudaGetLastError());
                 plan->launches += 2;
             }
